@@ -4,26 +4,43 @@
 //   popcount(F[p] ^ M[clamp(p + d(label))]),
 // d(label) = (ly, lx, lz) * q - q*hw, label = ly + lx*len + lz*len^2.
 //
-// Main path (grid spacing 2..8): the moving codes are first copied into a
-// clamp-to-edge padded volume (the reference's data2p, :124-138), with an even
-// row pitch so that every row is 16-byte aligned for TMA.  One CTA owns a tile
-// of NY consecutive control nodes along y (same x, z) and one z label offset lz;
-// it walks the len x-offsets lx.  For each (lx, lz) the halo it needs is one 3-D
-// box of the padded volume — all y rows of the tile plus the label reach, the
-// sampled x columns and z slices — which a single cp.async.bulk.tensor.3d
-// copies into shared memory (element strides 2 in x and z skip the unsampled
-// columns, as the reference's skipx/skipz do).  Two boxes are in flight
-// (double buffering on two mbarriers).  Threads own one (node, ly) label each
-// and reduce the node's samples with fully unrolled loops: per sample one
-// 64-bit shared load of the moving code and an XOR with the fixed code (held in
-// registers); three samples' XORs go through a carry-save adder so that they cost
-// two 64-bit POPCs instead of three.
-// NY is chosen per level by the autotuner in pipeline.cpp.
+// Main path (grid spacing 2..8): the sums run on the tensor cores, as dot products
+// of 64 four-bit floats (E2M1) per code whose terms are bit differences less a
+// constant of the fixed code (tmem_st_moving, expand_fixed); a row's sums over its
+// node's sampled columns accumulate exactly in the fp32 accumulators (multiples of
+// 1/2 of at most 2^11).
 //
-// Roofline: integer-pipe bound (32-bit POPCs: GB300 issues 16 per clock per SM;
-// four per three 64-bit samples with the carry-save adder, against two per sample
-// in the XOR + POPC probe).  Work per launch = sz1 * len^3 * samples popc64.
-#include <cuda.h>
+// A label step of q pairs only rows y of one residue modulo q, so rows are taken
+// by residue class: class r of a tile of tn nodes along y (one x, z) has the fixed
+// rows r + q a and the moving rows r + q b, and y label ly pairs b = a + ly.  With
+// a0 = floor(t G / q), node t's fixed rows of any class are a = a0 + s for slots
+// s < SL = ceil((G + q - 1) / q) at most, and (t, s, b) stands for the label
+// ly = b - a0 - s in every class.  One step of work = (P z offsets, x offset lx) is
+//   D[(p, b)][(t, s)] += <moving rows of class r, fixed rows of class r>
+// over the node's sampled columns and the q classes, M = 128 moving rows (P offsets
+// x R rows) by N >= tn SL slots, all in the accumulators; a label's cost is the sum
+// of its SL entries.
+//  * three producer warpgroups (classes in turn): one thread per moving row loads
+//    its codes (from a copy of the volume with its rows split by class, so that
+//    loads are contiguous), expands them in registers and stores them to tensor
+//    memory as operand A: a ring of twelve x columns, of which a step shares all but
+//    one with the step before where q is 1;
+//  * two warps (steps in turn) issue tcgen05.mma.kind::mxf4 with unit scales; operand
+//    B = the fixed rows, expanded once per CTA into shared memory;
+//  * two epilogue warpgroups (steps in turn; three where the window slides) move the
+//    accumulators to shared memory and sum the slots.
+//
+// Bound: of a step's products len P T in 128 N are used, and an MMA costs max(15,
+// N / 2) clocks per column with operand A in tensor memory (max(39, 32 + N / 4) from
+// shared memory): 25-47 useful code pairs a clock and SM, where the integer pipe does
+// 12 (four 32-bit POPCs per three pairs with a carry-save adder) and the kernel that
+// used it reached 7.5.  Reached: 13-20 (the tensor pipe is busy 43 % of the time at
+// grid 8): issuing an MMA takes ~32 clocks and each class ~320 for the hand-overs
+// between the warps.  192x160x256, one direction, grids 8/7/6/5/4 of the default
+// schedule: 1.89 / 1.39 / 1.30 / 1.56 / 1.37 ms, 7.5 ms in all (13.8 ms on the integer
+// pipe); a 131x118x141 level of grid 5, radius 4, step 3: 0.65 -> 0.24 ms.
+#include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -32,193 +49,439 @@ namespace deeds {
 
 namespace {
 
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2) {
+// ---- tensor memory and block-scaled 4-bit MMA (one CTA)
+__device__ __forceinline__ void tmem_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tmem_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_st8(uint32_t addr, const uint32_t (&w)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(addr), "r"(w[0]),
+                 "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t addr, float (&v)[16]) {
     asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-        ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, "
+        "[%16];"
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]),
+          "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15])
+        : "r"(addr)
         : "memory");
 }
-
-// clamp-to-edge padded copy of the moving codes, row pitch mpp (even)
-__global__ void k_pad_codes(const uint64_t* __restrict__ M, uint64_t* __restrict__ Mp, int m, int n, int o, int pad,
-                            int mpp, int np, int op) {
-    const int y = blockIdx.x * blockDim.x + threadIdx.x;
-    const int x = blockIdx.y, z = blockIdx.z;
-    if (y >= mpp) return;
-    const int64_t src = clampi(y - pad, 0, m - 1) + (int64_t)clampi(x - pad, 0, n - 1) * m +
-                        (int64_t)clampi(z - pad, 0, o - 1) * m * n;
-    Mp[y + (int64_t)x * mpp + (int64_t)z * mpp * np] = __ldg(M + src);
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t p;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(p));
+    return p;
+}
+// D[128][N] (+)= A[128][64] B[N][64]: A in tensor memory (lane = row, eight 4-bit
+// elements per column word), B in shared memory
+template <bool FIRST>  // FIRST: where `more` is 0 the product replaces D
+__device__ __forceinline__ void mma_mxf4(uint32_t d, uint32_t a, uint32_t blo, uint32_t bhi, uint32_t idesc, uint32_t sfa,
+                                         uint32_t sfb, uint32_t more) {
+    asm volatile(
+        "{\n .reg .pred p;\n .reg .b64 b;\n mov.b64 b, {%2, %3};\n setp.ne.u32 p, %7, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], [%1], b, %4, [%5], [%6], p;\n}" ::"r"(d),
+        "r"(a), "r"(blo), "r"(bhi), "r"(idesc), "r"(sfa), "r"(sfb), "r"(FIRST ? more : 1u)
+        : "memory");
+}
+__device__ __forceinline__ void mma_commit(uint64_t* bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
+                 : "memory");
+}
+__device__ __forceinline__ void st_shared(uint32_t at, float v) {
+    asm volatile("st.shared.f32 [%0], %1;" ::"r"(at), "f"(v) : "memory");
+}
+// Wait for an mbarrier phase with the hardware's own short suspension (a suspend-time
+// hint polls, which took a third of the issue slots here).  Bounded by the number of
+// tries, under a microsecond each: the time a preempted context spends off the GPU
+// does not count.
+constexpr uint32_t kTries = 1u << 22;
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
+    const uint32_t at = smem_u32(bar);
+    for (uint32_t i = 0; i < kTries; i++) {
+        uint32_t ok;
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+            : "=r"(ok)
+            : "r"(at), "r"(parity)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// true if any of the `count` threads on named barrier `id` passes true
+__device__ __forceinline__ bool bar_any(int id, int count, bool v) {
+    uint32_t r;
+    asm volatile(
+        "{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n bar.red.or.pred q, %2, %3, p;\n selp.u32 %0, 1, 0, q;\n}"
+        : "=r"(r)
+        : "r"((uint32_t)v), "r"(id), "r"(count)
+        : "memory");
+    return r != 0;
 }
 
-// Sum of the G sample-row partials of tile node t at label ly into its cost entry.
-template <int G>
-__device__ __forceinline__ void reduce_rows(const int* red, int nthr, int t, int ly, float* cost_lx, int len3,
-                                            float alpha1) {
-    const int* r = red + ly * nthr + t * G;
-    int sum = 0;
+// A code's 64 bits as 4-bit floats, nibble by nibble of its two words.  Each moving
+// bit is used where it stands in its nibble, as 0.5, 1, 2 (bits 0, 1, 2) or as a
+// sign (bit 3), so that a word costs one logic operation; the fixed code supplies
+// the factor that makes the product of bit m and bit f
+//   m (1 - 2 f) = (m ^ f) - f        (bits 0, 1, 2: factors +-2, +-1, +-1/2)
+//   -(1 - 2 m)(1 - 2 f) / 2 = (m ^ f) - 1/2   (bit 3: the sign times -+1/2)
+// so a code pair's dot product is popcount(m ^ f) - fixed_term(f).
+__device__ __forceinline__ void tmem_st_moving(uint32_t addr, uint64_t c) {
+    asm volatile(
+        "{\n .reg .b32 w<8>;\n"
+        " and.b32 w0, %1, 0x11111111;\n and.b32 w1, %1, 0x22222222;\n and.b32 w2, %1, 0x44444444;\n"
+        " lop3.b32 w3, %1, 0x88888888, 0x22222222, 0xea;\n"
+        " and.b32 w4, %2, 0x11111111;\n and.b32 w5, %2, 0x22222222;\n and.b32 w6, %2, 0x44444444;\n"
+        " lop3.b32 w7, %2, 0x88888888, 0x22222222, 0xea;\n"
+        " tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {w0, w1, w2, w3, w4, w5, w6, w7};\n}" ::"r"(addr),
+        "r"((uint32_t)c), "r"((uint32_t)(c >> 32))
+        : "memory");
+}
+__device__ __forceinline__ void expand_fixed(uint64_t c, uint32_t (&w)[8]) {
 #pragma unroll
-    for (int ii = 0; ii < G; ii++) sum += r[ii];
-    cost_lx[(int64_t)t * len3 + ly] = __fmul_rn((float)sum, alpha1);
+    for (int h = 0; h < 2; h++) {
+        const uint32_t v = (uint32_t)(c >> (32 * h));
+        w[4 * h + 0] = ((v << 3) & 0x88888888u) | 0x44444444u;
+        w[4 * h + 1] = ((v << 2) & 0x88888888u) | 0x22222222u;
+        w[4 * h + 2] = ((v << 1) & 0x88888888u) | 0x11111111u;
+        w[4 * h + 3] = (v & 0x88888888u) ^ 0x99999999u;
+    }
+}
+__device__ __forceinline__ int fixed_term(uint64_t c) { return __popcll(c & 0x7777777777777777ull) + 8; }
+
+// Producer and epilogue warpgroups: a sliding window expands a quarter of the codes
+// per step and finishes as many labels, so it has one more epilogue warpgroup.
+constexpr int kGroups = 5;
+constexpr int epi_groups(bool slide) { return slide ? 3 : 2; }
+constexpr int kMmaWarp = 4 * kGroups;
+constexpr int kCostThreads = (kMmaWarp + 2) * 32;
+constexpr int kRingCols = 12;  // x columns of operand A in tensor memory
+constexpr int kDCols = 96;     // columns of all accumulators: one per epilogue warpgroup
+constexpr int kEntryPitch = 132;  // entries [slot][128 moving rows]: neighbouring nodes' slots start in different banks
+constexpr uint32_t kColD = 384, kColS = 480;  // tensor memory columns: A ring | 2 accumulators | scales
+
+// How a level's labels are cut into tiles (cost_plan).
+struct CostPlan {
+    int tn, SL;  // nodes per tile along y, slots per node
+    int N;       // tn SL rounded up to 16
+    int P, R;    // z offsets per step, moving rows of each: P R <= 128
+    int nly;     // y labels per chunk
+    int tiles_y, groups, groups_per_cta, splits, chunks;
+    int pitch;   // moving rows per class of the split copy
+};
+
+// The moving codes with each line's rows split by residue modulo q: class r, entry
+// b = row r + q b of the line padded by `pad` clamped rows in front.
+__global__ void k_split_rows(const uint64_t* __restrict__ M, uint64_t* __restrict__ Ms, int m, int n, int pad, int q,
+                             int pitch) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= q * pitch) return;
+    const int r = e / pitch, b = e - r * pitch;
+    const int64_t line = blockIdx.y + (int64_t)blockIdx.z * n;
+    Ms[line * q * pitch + e] = __ldg(M + line * m + clampi(r + q * b - pad, 0, m - 1));
 }
 
-// LEN_T/Q_T > 0: label width and quantisation fixed at compile time (the default
-// level schedule), so every label loop is exact and fully unrolled; 0: runtime
-// values, labels processed in chunks of 8 with guards.
-template <int G, int LEN_T, int Q_T>
-__global__ void __launch_bounds__(256) k_data_cost_tma(const __grid_constant__ CUtensorMap map,
-                                                       const uint64_t* __restrict__ F, float* __restrict__ cost,
-                                                       int m, int n, int o, int len_rt, int q_rt, int ny_tile, int yb,
-                                                       float alpha1, int* __restrict__ err) {
-    constexpr bool kFixed = LEN_T > 0;
-    const int len = kFixed ? LEN_T : len_rt;
-    const int q = kFixed ? Q_T : q_rt;
+// Ms: the split copy (q > 1) or the volume itself (q == 1, pitch 0).  SLIDE: a label
+// step of 1 with every sample taken, where a step's window moves by one x column.
+template <int G, bool SLIDE>
+__global__ void __launch_bounds__(kCostThreads, 1)
+    k_data_cost_mma(const uint64_t* __restrict__ F, const uint64_t* __restrict__ Ms, float* __restrict__ cost, int m,
+                    int n, int o, int len, int q, CostPlan pl, float alpha1, int* __restrict__ err) {
     constexpr int S = G > 4 ? 2 : 1;  // x and z sampling stride (RAND_SAMPLES=1, src/dataCostD.h:141-155)
-    constexpr int NX = (G + S - 1) / S, NZ = (G + S - 1) / S;
-    constexpr int NC = NX * NZ;       // sampled (x, z) columns per node
-    constexpr int CHUNK = 8;          // labels accumulated per pass over the columns
-    extern __shared__ __align__(128) uint64_t smem_raw[];
-    // TMA destinations must start on 128-byte boundaries: align explicitly
-    uint64_t* smem = reinterpret_cast<uint64_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~(uintptr_t)127);
-    __shared__ __align__(8) uint64_t bars[2];
-    __shared__ int s_ok;
-    const int box = NC * yb;
-    const int bstride = (box + 15) & ~15;
-    uint64_t* buf0 = smem;
-    uint64_t* buf1 = smem + bstride;
-    int* red = reinterpret_cast<int*>(smem + 2 * bstride);  // [len][threads] partial sums
-    const int m1 = m / G, n1 = n / G;
-    const int tiles_y = (m1 + ny_tile - 1) / ny_tile;
-    int b = blockIdx.x;
-    const int ty = b % tiles_y;
-    b /= tiles_y;
-    const int nxn = b % n1, nzn = b / n1;
-    const int lz = blockIdx.y;
-    const int y_first = ty * ny_tile;
-    const int ny_here = min(ny_tile, m1 - y_first);
-    const int y0 = y_first * G;  // padded y of the tile's first row (the pad offset cancels)
-    const int y_al = y0 & ~1;    // TMA: the innermost coordinate must be 16-byte aligned
-    const int yoff = y0 - y_al;
-    const int tid = threadIdx.x, nthr = blockDim.x;
+    constexpr int NX = (G + S - 1) / S, NZ = NX, NC = NX * NZ;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ __align__(8) uint64_t b_full[4], b_done[4], b_acc[3], b_free[3], b_turn[2];
+    __shared__ uint32_t s_tmem;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int len2 = len * len, len3 = len2 * len;
-    const int64_t mn = (int64_t)m * n;
-    const uint32_t box_bytes = (uint32_t)box * 8u;
-    const int xbase = nxn * G, zbase = nzn * G + lz * q;
-    if (tid == 0) {
-        mbar_init(&bars[0], 1);
-        mbar_init(&bars[1], 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        s_ok = 1;
+    const int m1 = m / G, n1 = n / G;
+    constexpr int kEpiGroups = epi_groups(SLIDE), kProdGroups = kGroups - kEpiGroups;
+    constexpr int kMaxN = kDCols / kEpiGroups;  // slots of a tile at most
+    constexpr int USTEP = SLIDE ? 1 : NX;  // new x columns per tile
+    // shared memory: B [class][column][2][N][16 B] | entries [2 warpgroups][N][kEntryPitch] | fixed terms [tn]
+    const uint32_t col_bytes = (uint32_t)pl.N * 32u;
+    float* entries = reinterpret_cast<float*>(smem_raw + (size_t)q * NC * col_bytes);
+    int* s_term = reinterpret_cast<int*>(entries + kEpiGroups * pl.N * kEntryPitch);
+    int b = blockIdx.x;
+    const int ty = b % pl.tiles_y;
+    b /= pl.tiles_y;
+    const int nxn = b % n1, nzn = b / n1;
+    const int g_first = blockIdx.y * pl.groups_per_cta;
+    const int n_groups = min(pl.groups_per_cta, pl.groups - g_first);
+    const int ly0 = blockIdx.z * pl.nly;
+    const int n_ly = min(pl.nly, len - ly0);
+    const int group_tiles = q * len, n_tiles = n_groups * group_tiles;
+    const int y_first = ty * pl.tn, y0 = y_first * G;
+    const int pad = q * (len - 1) / 2;
+    const int y0_q = y0 / q, y0_res = y0 - y0_q * q;
+
+    if (warp == kMmaWarp) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&s_tmem))
+                     : "memory");
+        if (lane == 0) {
+            for (int i = 0; i < 4; i++) {
+                mbar_init(&b_full[i], 4);
+                mbar_init(&b_done[i], 1);
+            }
+            for (int i = 0; i < kEpiGroups; i++) {
+                mbar_init(&b_acc[i], 1);
+                mbar_init(&b_free[i], 4);
+            }
+            for (int i = 0; i < 2; i++) mbar_init(&b_turn[i], 1);
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
     }
+    for (int e = tid; e < pl.tn; e += kCostThreads) s_term[e] = 0;
+    tmem_fence_before();
     __syncthreads();
-    if (tid == 0) {
-        mbar_expect_tx(&bars[0], box_bytes);
-        tma_load_3d(buf0, &map, &bars[0], y_al, xbase, zbase);
-        if (len > 1) {
-            mbar_expect_tx(&bars[1], box_bytes);
-            tma_load_3d(buf1, &map, &bars[1], y_al, xbase + q, zbase);
-        }
+    tmem_fence_after();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
+    if (warp < 4) {  // unit scales (E8M0 127) in every byte of the scale columns
+        const uint32_t one = 0x7f7f7f7fu;
+        const uint32_t w[8] = {one, one, one, one, one, one, one, one};
+        const uint32_t at = tmem + kColS + ((uint32_t)(warp * 32) << 16);
+        tmem_st8(at, w);
+        tmem_st8(at + 8, w);
+        tmem_wait_st();
     }
-    // this thread's node (within the tile) and sample row i: thread = node * G + i over
-    // the whole block, so a node's rows may straddle two warps and no lane idles
-    // but the last warp's tail; its fixed codes stay in registers
-    const int tn = tid / G, i = tid - (tid / G) * G;  // node index within the tile, sample row
-    const bool active = tn < ny_here;
-    uint64_t fr[NC];
-#pragma unroll
-    for (int c = 0; c < NC; c++) {
-        const int j = c % NX, k = c / NX;
-        fr[c] = active ? F[(y0 + tn * G + i) + (int64_t)(xbase + j * S) * m + (int64_t)(nzn * G + k * S) * mn] : 0ull;
+    // operand B: slot (t, s) of class r holds the fixed row f = r + q (a0 + s) where it is
+    // one of node t's, else zero
+    for (int e = tid; e < q * NC * pl.N; e += kCostThreads) {
+        const int rc = e / pl.N, a = e - rc * pl.N;
+        const int r = rc / NC, c = rc - r * NC;
+        const int t = a / pl.SL, f = r + q * (t * G / q + a - t * pl.SL), j = c % NX, k = c / NX;
+        uint32_t w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        if (t < pl.tn && f >= t * G && f < t * G + G && y0 + f < m) {
+            const uint64_t code = F[(y0 + f) + (int64_t)(nxn * G + j * S) * m + (int64_t)(nzn * G + k * S) * m * n];
+            expand_fixed(code, w);
+            atomicAdd(&s_term[t], fixed_term(code));
+        }
+        uint4* d = reinterpret_cast<uint4*>(smem_raw + (size_t)rc * col_bytes + a * 16);
+        d[0] = make_uint4(w[0], w[1], w[2], w[3]);
+        d[pl.N] = make_uint4(w[4], w[5], w[6], w[7]);
     }
-    const int pos = yoff + tn * G + i;  // this thread's row in the box (for label ly add ly*q)
-    // partial sums: [warp][len][32] when g divides 32 (the warp reduces its own
-    // nodes), else [len][threads] (nodes straddle warps: the block reduces)
-    constexpr bool kWarpLocal = 32 % G == 0;
-    int* wred = kWarpLocal ? red + (tid >> 5) * len * 32 + (tid & 31) : red + tid;
-    const int wstride = kWarpLocal ? 32 : nthr;
-    for (int lx = 0; lx < len; lx++) {
-        const int slot = lx & 1;
-        const uint64_t* sb = slot ? buf1 : buf0;
-        if (tid == 0) {
-            if (!mbar_wait_bounded(&bars[slot], (uint32_t)((lx >> 1) & 1))) s_ok = 0;
-        }
-        __syncthreads();
-        if (!s_ok) break;
-        if (kFixed && active) {
-            constexpr int LF = kFixed ? LEN_T : 1, QF = kFixed ? Q_T : 1;
-            int acc[LF];
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    tmem_fence_before();
+    __syncthreads();
+    tmem_fence_after();
+
+    const auto wait_done = [&](int t) { return mbar_wait(&b_done[t & 3], (uint32_t)((t >> 2) & 1)); };
+    const auto wait_full = [&](int t) { return mbar_wait(&b_full[t & 3], (uint32_t)((t >> 2) & 1)); };
+    const uint32_t quadrant = (uint32_t)((warp & 3) * 32) << 16;
+    const int row = tid & 127;
+    const int p = row / pl.R, yb = row - p * pl.R;  // this thread's z offset and moving row
+    bool ok = true;
+    if (warp < 4 * kProdGroups) {
+        // ---- producers
+        const int wg = warp >> 2;
+        const uint32_t line = q > 1 ? (uint32_t)(q * pl.pitch) : (uint32_t)m;
+        // a row's place in its line: entry y0 / q + ly0 + yb of a class, or the clamped row
+        const uint32_t at = q > 1 ? (uint32_t)(ly0 + yb) : (uint32_t)clampi(y0 + ly0 + yb - pad, 0, m - 1);
+        uint32_t zo[NZ];  // this thread's place in the volume less the x offset (below 2^32: cost_plan)
+        uint64_t code[NX][NZ];
+        // the tile to load next: class r, x offset lx of group gi; x = tile of the group
+        int r = 0, lx = 0, gi = 0, x = 0, col = 0;  // col: its first ring column
+        auto next = [&]() {
+            if (++r == q) { r = 0; lx++; }
+            col += USTEP;
+            if (++x == group_tiles) { x = 0; lx = 0; gi++; col += NX - USTEP; }
+            if (col >= kRingCols) col -= kRingCols;
+        };
+        for (int i = 0; i < wg; i++) next();
+        int group_set = -1;
+        auto load = [&]() {
+            if (gi != group_set) {
+                group_set = gi;
+                const int lz = (g_first + gi) * pl.P + p;
 #pragma unroll
-            for (int u = 0; u < LF; u++) acc[u] = 0;
-            // samples three at a time through a carry-save adder: for the XORs a, b, c,
-            // popc(a) + popc(b) + popc(c) = popc(a ^ b ^ c) + 2 popc(maj(a, b, c)), two
-            // 64-bit POPCs (the kernel's bound: 16 per clock per SM) instead of three
+                for (int k = 0; k < NZ; k++)
+                    zo[k] = at + (uint32_t)clampi(nzn * G + k * S + lz * q - pad, 0, o - 1) * (uint32_t)n * line;
+            }
+            const int cls = y0_res + r >= q ? y0_res + r - q : y0_res + r;
+            const uint32_t off = q > 1 ? (uint32_t)(cls * pl.pitch + y0_q + (y0_res + r >= q)) : 0u;
 #pragma unroll
-            for (int c = 0; c + 3 <= NC; c += 3) {
-                const uint64_t* ca = sb + c * yb + pos;
-                const uint64_t* cb = ca + yb;
-                const uint64_t* cc = cb + yb;
+            for (int j = 0; j < NX; j++) {
+                if (SLIDE && x > 0 && j < NX - 1) continue;  // the column is in the ring
+                const uint64_t* src = Ms + ((uint32_t)clampi(nxn * G + j * S + lx * q - pad, 0, n - 1) * line + off);
 #pragma unroll
-                for (int u = 0; u < LF; u++) {
-                    const uint64_t a = fr[c] ^ ca[u * QF], b = fr[c + 1] ^ cb[u * QF], x = fr[c + 2] ^ cc[u * QF];
-                    const uint64_t sum = a ^ b ^ x, carry = (a & b) | (x & (a ^ b));
-                    acc[u] += __popcll(sum) + 2 * __popcll(carry);
+                for (int k = 0; k < NZ; k++) code[j][k] = __ldg(src + zo[k]);
+            }
+        };
+        if (wg < n_tiles) load();
+        for (int t = wg; t < n_tiles; t += kProdGroups) {
+            // the columns overwritten were last read by tile t - 3 or before: a tile
+            // moves the ring by at most NX <= 4 of its 12 columns.  (Every tile's phase is
+            // waited for in turn: a parity says nothing about the phase before it.)
+            for (int d = kProdGroups + 2; d >= 3 && ok; d--)
+                if (t >= d) ok = wait_done(t - d);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            tmem_fence_after();
+            int cj = col;
+#pragma unroll
+            for (int j = 0; j < NX; j++) {
+                if (!SLIDE || x == 0 || j == NX - 1) {
+                    const uint32_t to = tmem + quadrant + (uint32_t)(cj * NZ * 8);
+#pragma unroll
+                    for (int k = 0; k < NZ; k++) tmem_st_moving(to + k * 8, code[j][k]);
                 }
+                cj = cj + 1 == kRingCols ? 0 : cj + 1;
             }
-#pragma unroll
-            for (int c = NC - NC % 3; c < NC; c++) {
-                const uint64_t* col = sb + c * yb + pos;
-#pragma unroll
-                for (int u = 0; u < LF; u++) acc[u] += __popcll(fr[c] ^ col[u * QF]);
-            }
-#pragma unroll
-            for (int u = 0; u < LF; u++) wred[u * wstride] = acc[u];
-        } else if (active) {
-            for (int ly0 = 0; ly0 < len; ly0 += CHUNK) {
-                int acc[CHUNK];
-#pragma unroll
-                for (int u = 0; u < CHUNK; u++) acc[u] = 0;
-#pragma unroll
-                for (int c = 0; c < NC; c++) {
-                    const uint64_t* col = sb + c * yb + pos + ly0 * q;
-#pragma unroll
-                    for (int u = 0; u < CHUNK; u++)
-                        if (ly0 + u < len) acc[u] += __popcll(fr[c] ^ col[u * q]);
-                }
-#pragma unroll
-                for (int u = 0; u < CHUNK; u++)
-                    if (ly0 + u < len) wred[(ly0 + u) * wstride] = acc[u];
-            }
-        }
-        // sum the G sample rows of each (node, ly): within the warp when g divides 32
-        // (no node straddles two warps), else over the block
-        // (cost row of tile node t, label ly): node (y_first + t) + nxn m1 + nzn m1 n1
-        float* cost_lx = cost + (int64_t)(y_first + nxn * m1 + nzn * m1 * n1) * len3 + lx * len + lz * len2;
-        if constexpr (kWarpLocal) {
-            constexpr int WN = 32 / G;  // nodes per warp
+            for (int i = 0; i < kProdGroups; i++) next();
+            if (t + kProdGroups < n_tiles) load();
+            tmem_wait_st();
+            tmem_fence_before();
             __syncwarp();
-            const int warp = tid >> 5, lane = tid & 31;
-            const int* wr = red + warp * len * 32;
-            for (int e = lane; e < WN * len; e += 32) {
-                const int en = e / len, node_t = warp * WN + en;
-                if (node_t < ny_here) reduce_rows<G>(wr, 32, en, e - en * len, cost_lx + (int64_t)warp * WN * len3, len3,
-                                                     alpha1);
+            if (lane == 0) mbar_arrive(&b_full[t & 3]);
+        }
+    } else if (warp < kMmaWarp) {
+        // ---- epilogue: warpgroup e takes steps e, e + kEpiGroups, ... from accumulator e
+        const int e = (warp >> 2) - kProdGroups;
+        const uint32_t acc = tmem + kColD + (uint32_t)(e * kMaxN) + quadrant;
+        float* const mine = entries + e * pl.N * kEntryPitch;
+        const uint32_t at = smem_u32(mine) + 4u * (uint32_t)row;
+        const int ny_here = min(pl.tn, m1 - y_first);
+        // this thread's sums: kSums at most in registers, others recomputed
+        constexpr int kSums = 5;
+        const int outputs = pl.P * pl.tn * pl.nly;
+        int s_at[kSums], s_out[kSums], s_k[kSums];  // first entry, cost entry (-1: none), fixed term
+        auto sum_of = [&](int x, int& from, int& to, int& term) {
+            const int a = x / pl.nly, ly = x - a * pl.nly;  // x = (pp tn + node) nly + ly
+            const int pp = a / pl.tn, node = a - pp * pl.tn;
+            from = node * pl.SL * kEntryPitch + pp * pl.R + node * G / q + ly;
+            to = x < outputs && node < ny_here && ly < n_ly ? node * len3 + pp * len2 + ly : -1;
+            term = x < outputs ? s_term[node] : 0;
+        };
+#pragma unroll
+        for (int i = 0; i < kSums; i++) sum_of(row + i * 128, s_at[i], s_out[i], s_k[i]);
+        float* const cost0 = cost + (int64_t)(y_first + nxn * m1 + nzn * m1 * n1) * len3 + ly0;
+        const int n_steps = n_groups * len;
+        int lx = e, gi = 0;
+        while (lx >= len) { lx -= len; gi++; }
+        for (int st = e; st < n_steps; st += kEpiGroups) {
+            ok = __all_sync(0xffffffffu, mbar_wait(&b_acc[e], (uint32_t)((st / kEpiGroups) & 1)));
+            if (ok) {
+                tmem_fence_after();
+#pragma unroll
+                for (int c = 0; c < kMaxN; c += 16) {
+                    if (c >= pl.N) break;
+                    float v[16];
+                    tmem_ld16(acc + c, v);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int u = 0; u < 16; u++) st_shared(at + 4 * (c + u) * kEntryPitch, v[u]);
+                }
+                tmem_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&b_free[e]);
             }
-        } else {
-            __syncthreads();
-            for (int e = tid; e < ny_here * len; e += nthr)
-                reduce_rows<G>(red, nthr, e / len, e - (e / len) * len, cost_lx, len3, alpha1);
+            if (bar_any(1 + e, 128, !ok)) { ok = false; break; }
+            const int lz0 = (g_first + gi) * pl.P;
+            float* ct = cost0 + lx * len + lz0 * len2;
+            auto emit = [&](int from, int to, int term) {
+                float sum = (float)term;  // popcount = the entries + the fixed terms, exact
+                #pragma unroll
+                for (int i = 0; i < G; i++)
+                    if (i < pl.SL) sum += mine[from + i * (kEntryPitch + 1)];
+                ct[to] = __fmul_rn(sum, alpha1);
+            };
+            const bool whole = lz0 + pl.P <= len;  // the last group may have fewer z offsets
+            if (whole) {
+#pragma unroll
+                for (int i = 0; i < kSums; i++)
+                    if (s_out[i] >= 0) emit(s_at[i], s_out[i], s_k[i]);
+            }
+            for (int x = row + (whole ? kSums * 128 : 0); x < outputs; x += 128) {
+                int from, to, term;
+                sum_of(x, from, to, term);
+                if (to >= 0 && lz0 + to % len3 / len2 < len) emit(from, to, term);
+            }
+            bar_any(1 + e, 128, false);  // the entries are read
+            lx += kEpiGroups;
+            while (lx >= len) { lx -= len; gi++; }
         }
-        __syncthreads();  // every thread is done with this buffer and with red
-        if (tid == 0 && lx + 2 < len) {
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            mbar_expect_tx(&bars[slot], box_bytes);
-            tma_load_3d(const_cast<uint64_t*>(sb), &map, &bars[slot], y_al, xbase + (lx + 2) * q, zbase);
+    } else {
+        // ---- MMA warps: warp e issues steps e, e + 2, ... into the accumulators in turn
+        // (e a constant of each copy: the operands' arithmetic stays uniform)
+        const auto issue_steps = [&](auto which) {
+        constexpr int e = decltype(which)::value;
+        const uint32_t el = elect_one();
+        // M = 128, N, E2M1 operands, E8M0 scales, K = 64
+        const uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(pl.N >> 3) << 17) | (1u << 23) | (1u << 27);
+        // B: K-major without swizzle: 8 x 16 B core matrices, 128 B apart along the
+        // rows, N * 16 B apart along K
+        const uint32_t blo0 = ((smem_u32(smem_raw) & 0x3ffffu) >> 4) | ((uint32_t)pl.N << 16);
+        const uint32_t bhi = 8u | (1u << 14), sf = tmem + kColS;
+        int last = -1;  // the last step committed
+        const int n_steps = n_groups * len;
+        int x = 0, col = 0;  // the step's number in its group, its first ring column
+        const auto next = [&]() {
+            col += q * USTEP;
+            if (++x == len) { x = 0; col += NX - USTEP; }
+            col %= kRingCols;
+        };
+        if (e) next();
+        for (int st = e; st < n_steps; st += 2) {
+            // (A wait that gives up only marks the launch as failed: the warp goes on without a
+            // branch, so that the operands stay in uniform registers and the issue does not stall.)
+            bool in = true;
+            // the other warp has seen every tile of its step in place, and its accumulator
+            // free (a parity says nothing about the phase before it)
+            if (st >= 1) in = mbar_wait(&b_turn[1 - e], (uint32_t)(((st - 1) >> 1) & 1));
+            const int acc = st % kEpiGroups;
+            if (st >= kEpiGroups) in = in && mbar_wait(&b_free[acc], (uint32_t)((st / kEpiGroups - 1) & 1));
+            const uint32_t d = tmem + kColD + (uint32_t)(acc * kMaxN);
+            ok = ok && in;
+            int cj = col;
+            uint32_t blo = blo0;
+            for (int r = 0; r < q; r++) {
+                const int t = st * q + r;
+                ok = wait_full(t) && ok;
+                if (r == q - 1 && lane == 0) mbar_arrive(&b_turn[e]);
+                tmem_fence_after();
+                if (el) {
+#pragma unroll
+                    for (int j = 0; j < NX; j++) {
+                        int c = cj + j;
+                        c = c >= kRingCols ? c - kRingCols : c;
+                        const uint32_t a = tmem + (uint32_t)(c * NZ * 8);
+#pragma unroll
+                        for (int k = 0; k < NZ; k++) {
+                            const uint32_t bl = blo + (uint32_t)(k * NX + j) * (col_bytes >> 4);
+                            if (j + k == 0) mma_mxf4<true>(d, a, bl, bhi, idesc, sf, sf + 8, (uint32_t)r);
+                            else mma_mxf4<false>(d, a + k * 8, bl, bhi, idesc, sf, sf + 8, 1u);
+                        }
+                    }
+                    mma_commit(&b_done[t & 3]);
+                    if (r == q - 1) mma_commit(&b_acc[acc]);
+                }
+                __syncwarp();
+                cj += NX;
+                cj = cj >= kRingCols ? cj - kRingCols : cj;
+                blo += (uint32_t)NC * (col_bytes >> 4);
+                last = st;
+            }
+            next();
+            next();
         }
+        // no MMA is in flight when the memory is given back: its commits have arrived
+        // (each warp waits for its own last one)
+        if (last >= 0 && !mbar_wait(&b_acc[last % kEpiGroups], (uint32_t)((last / kEpiGroups) & 1))) ok = false;
+        };
+        if (warp == kMmaWarp) issue_steps(std::integral_constant<int, 0>{});
+        else issue_steps(std::integral_constant<int, 1>{});
     }
-    if (!s_ok && tid == 0) {
-        atomicCAS(err, 0, 3);
-        // wait (bounded) for the copies this CTA may still have in flight
-        for (int sl = 0; sl < 2; sl++)
-            for (int ph = 0; ph < 2; ph++) mbar_wait_bounded(&bars[sl], (uint32_t)ph);
+    if (!ok) atomicCAS(err, 0, 3);
+    tmem_fence_before();
+    __syncthreads();
+    if (warp == kMmaWarp) {
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
     }
 }
 
@@ -257,119 +520,110 @@ __global__ void __launch_bounds__(256) k_data_cost(const uint64_t* __restrict__ 
     }
 }
 
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        tried = true;
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) ==
-                cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(p);
-        cudaGetLastError();
-    }
-    return fn;
-}
-
-// threads of a cost-volume block: one per (node, sample row) of the tile, whole warps
-int data_cost_tma_threads(int g, int ny_tile) { return (ny_tile * g + 31) / 32 * 32; }
-
-size_t data_cost_tma_smem(int g, int hw, int q, int ny_tile) {
+size_t cost_smem(const CostPlan& c, int g, int q) {
     const int S = g > 4 ? 2 : 1, NX = (g + S - 1) / S;
-    const int len = 2 * hw + 1;
-    const int yb = ((ny_tile * g + (len - 1) * q + 1) + 1) & ~1;
-    return (size_t)2 * ((NX * NX * yb + 15) & ~15) * 8 + (size_t)data_cost_tma_threads(g, ny_tile) * len * 4 + 128;
+    return (size_t)q * NX * NX * c.N * 32 + (size_t)epi_groups(q == 1 && g <= 4) * c.N * kEntryPitch * 4 + (size_t)c.tn * 4;
 }
 
-template <int G, int LEN_T, int Q_T>
-cudaError_t launch_tma(const uint64_t* d_F, const uint64_t* d_Mp, int mpp, int np, int op, int m, int n, int o,
-                       int hw, int q, int ny_tile, float alpha1, float* d_cost, int* d_err, cudaStream_t s) {
-    constexpr int S = G > 4 ? 2 : 1;
-    constexpr int NX = (G + S - 1) / S, NZ = (G + S - 1) / S;
-    const int len = 2 * hw + 1;
-    const int yb = ((ny_tile * G + (len - 1) * q + 1) + 1) & ~1;  // +1 for the alignment shift, rounded to even
-    CUtensorMap map;
-    const cuuint64_t dims[3] = {(cuuint64_t)mpp, (cuuint64_t)np, (cuuint64_t)op};
-    const cuuint64_t strides[2] = {(cuuint64_t)mpp * 8, (cuuint64_t)mpp * np * 8};
-    const cuuint32_t boxd[3] = {(cuuint32_t)yb, (cuuint32_t)(NX * S), (cuuint32_t)(NZ * S)};
-    const cuuint32_t estr[3] = {1, (cuuint32_t)S, (cuuint32_t)S};
-    EncodeTiledFn enc = encode_fn();
-    if (!enc) return cudaErrorNotSupported;
-    if (enc(&map, CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, const_cast<uint64_t*>(d_Mp), dims, strides, boxd, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return cudaErrorInvalidValue;
-    const int threads = data_cost_tma_threads(G, ny_tile);
-    const size_t smem = data_cost_tma_smem(G, hw, q, ny_tile);
-    cudaError_t e =
-        cudaFuncSetAttribute(k_data_cost_tma<G, LEN_T, Q_T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+// The tile that makes a level cheapest, in clocks.  Measured per class: 33 per MMA
+// (its issue; N / 2 above N = 64) and 320 for the hand-overs; with a sliding window
+// the two issuing warps overlap.  A step's epilogue: 16 per slot, 270 per 128 sums.
+// A CTA's start: 3500 and the fixed rows.
+bool cost_plan(int m, int n, int o, int g, int len, int q, CostPlan& best) {
+    if (g < 2 || g > 8 || len < 3 || q < 1 || q > 64) return false;
+    const int S = g > 4 ? 2 : 1, NX = (g + S - 1) / S, NC = NX * NX;
+    const int m1 = m / g, n1 = n / g, o1 = o / g;
+    const int ustep = q == 1 && S == 1 ? 1 : NX;
+    // y labels per chunk: all of them unless they alone exceed the 128 rows
+    int chunks = 1;
+    while ((len + chunks - 1) / chunks - 1 + (g + q - 1) / q > 128) chunks++;
+    const int nly = (len + chunks - 1) / chunks;
+    chunks = (len + nly - 1) / nly;
+    double best_t = 1e300;
+    for (int tn = 1; tn <= m1; tn++) {
+        CostPlan c{};
+        c.tiles_y = (m1 + tn - 1) / tn;
+        if (tn > 1 && (m1 + tn - 2) / (tn - 1) == c.tiles_y) continue;  // fewer rows give the same tile count
+        c.tn = tn;
+        c.SL = (g + q - 1 + q - 1) / q;
+        if (g % q == 0) c.SL = g / q;
+        c.N = (tn * c.SL + 15) / 16 * 16;
+        c.R = (tn - 1) * g / q + c.SL + nly - 1;
+        c.nly = nly;
+        c.chunks = chunks;
+        if (c.N > kDCols / epi_groups(q == 1 && g <= 4) || c.R > 128) break;
+        for (c.P = 1; c.P * c.R <= 128 && c.P <= len; c.P++) {
+            c.groups = (len + c.P - 1) / c.P;
+            if (c.P > 1 && c.groups == (len + c.P - 2) / (c.P - 1)) continue;
+            if (cost_smem(c, g, q) > 200 * 1024) continue;
+            const bool slide = q == 1 && g <= 4;
+            const double rounds = (c.P * tn * nly + 127) / 128;
+            const double mma = slide ? NC * 22.0 + 350.0 : q * (NC * 33.0 + 320.0);
+            const double epi = (250.0 + 16.0 * c.N + 270.0 * rounds) / epi_groups(slide);
+            const double start = 3500.0 + q * NC * c.N * 0.8;
+            const double t = (std::max(mma, epi) * len * c.groups + start) * c.tiles_y;
+            if (t < best_t) {
+                best_t = t;
+                best = c;
+            }
+        }
+    }
+    if (best_t == 1e300) return false;
+    // rows per class: the last tile's rows (beyond the volume too) and the label reach
+    best.pitch = q > 1 ? (best.tiles_y * best.tn * g + q - 1) / q + chunks * nly + 2 : 0;
+    if ((uint64_t)std::max(m, q * best.pitch) * n * o >= (1ull << 32)) return false;
+    // enough CTAs for several waves of one per SM
+    const int64_t cols = (int64_t)best.tiles_y * n1 * o1 * chunks;
+    int splits = 1;
+    while (splits < best.groups && cols * splits < 8 * 152) splits++;
+    best.groups_per_cta = (best.groups + splits - 1) / splits;
+    best.splits = (best.groups + best.groups_per_cta - 1) / best.groups_per_cta;
+    return true;
+}
+
+template <int G, bool SLIDE>
+cudaError_t launch_mma(const uint64_t* d_F, const uint64_t* d_Ms, int m, int n, int o, int len, int q,
+                       const CostPlan& pl, float alpha1, float* d_cost, int* d_err, cudaStream_t s) {
+    const size_t smem = cost_smem(pl, G, q);
+    cudaError_t e = cudaFuncSetAttribute(k_data_cost_mma<G, SLIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    const int m1 = m / G, n1 = n / G, o1 = o / G;
-    const int tiles_y = (m1 + ny_tile - 1) / ny_tile;
-    dim3 grid((unsigned)(tiles_y * n1 * o1), (unsigned)len);
-    k_data_cost_tma<G, LEN_T, Q_T><<<grid, threads, smem, s>>>(map, d_F, d_cost, m, n, o, len, q, ny_tile, yb,
-                                                                   alpha1, d_err);
+    const dim3 grid((unsigned)(pl.tiles_y * (n / G) * (o / G)), (unsigned)pl.splits, (unsigned)pl.chunks);
+    k_data_cost_mma<G, SLIDE><<<grid, kCostThreads, smem, s>>>(d_F, d_Ms, d_cost, m, n, o, len, q, pl, alpha1, d_err);
     count_launches(1);
     return cudaGetLastError();
 }
 
 }  // namespace
 
-bool data_cost_tma_supported(int g, int hw, int q, int ny_tile) {
-    if (g < 2 || g > 8 || ny_tile < 1) return false;
+size_t data_cost_split_count(int m, int n, int o, int g, int hw, int q) {
+    CostPlan pl;
+    return cost_plan(m, n, o, g, 2 * hw + 1, q, pl) ? (size_t)pl.pitch * q * n * o : 0;
+}
+
+cudaError_t launch_data_cost_mma(const uint64_t* d_F, const uint64_t* d_M, uint64_t* d_split, int m, int n, int o,
+                                 int g, int hw, int q, float alpha1, float* d_cost, int* d_err, cudaStream_t s,
+                                 bool* taken) {
+    CostPlan pl;
     const int len = 2 * hw + 1;
-    if (data_cost_tma_threads(g, ny_tile) > 256) return false;
-    const int yb = ((ny_tile * g + (len - 1) * q + 1) + 1) & ~1;
-    if (yb > 256) return false;
-    return data_cost_tma_smem(g, hw, q, ny_tile) <= 200 * 1024 && encode_fn() != nullptr;
-}
-
-size_t padded_codes_count(int m, int n, int o, int pad) {
-    const size_t mpp = (size_t)((m + 2 * pad + 1) & ~1);
-    return mpp * (size_t)(n + 2 * pad) * (size_t)(o + 2 * pad);
-}
-
-cudaError_t launch_data_cost_tma(const uint64_t* d_F, const uint64_t* d_M, uint64_t* d_Mpad, int m, int n, int o,
-                                 int g, int hw, int q, int ny_tile, float alpha1, float* d_cost, int* d_err,
-                                 cudaStream_t s) {
-    const int pad = q * hw;
-    const int mpp = (m + 2 * pad + 1) & ~1, np = n + 2 * pad, op = o + 2 * pad;
-    {
-        dim3 blk(128), grd((mpp + 127) / 128, np, op);
-        k_pad_codes<<<grd, blk, 0, s>>>(d_M, d_Mpad, m, n, o, pad, mpp, np, op);
+    *taken = cost_plan(m, n, o, g, len, q, pl);
+    if (!*taken) return cudaSuccess;
+    const uint64_t* d_Ms = d_M;
+    if (q > 1) {
+        k_split_rows<<<dim3((q * pl.pitch + 127) / 128, n, o), 128, 0, s>>>(d_M, d_split, m, n, q * hw, q, pl.pitch);
         count_launches(1);
+        d_Ms = d_split;
     }
-    // deedsBCV's default level schedule (-G 8x7x6x5x4 -L 8x7x6x5x4 -Q 5x4x3x2x1) and
-    // linearBCV's have their own compile-time instantiations; everything else runs
-    // the runtime-width kernel
-#define DEEDS_TMA_ARGS d_F, d_Mpad, mpp, np, op, m, n, o, hw, q, ny_tile, alpha1, d_cost, d_err, s
-    if (g == 8 && hw == 8 && q == 5) return launch_tma<8, 17, 5>(DEEDS_TMA_ARGS);
-    if (g == 7 && hw == 7 && q == 4) return launch_tma<7, 15, 4>(DEEDS_TMA_ARGS);
-    if (g == 6 && hw == 6 && q == 3) return launch_tma<6, 13, 3>(DEEDS_TMA_ARGS);
-    if (g == 5 && hw == 5 && q == 2) return launch_tma<5, 11, 2>(DEEDS_TMA_ARGS);
-    if (g == 4 && hw == 4 && q == 1) return launch_tma<4, 9, 1>(DEEDS_TMA_ARGS);
-    // linearBCV's default schedule (src/linearBCV.cpp:86-89)
-    if (g == 7 && hw == 5 && q == 4) return launch_tma<7, 11, 4>(DEEDS_TMA_ARGS);
-    if (g == 6 && hw == 4 && q == 3) return launch_tma<6, 9, 3>(DEEDS_TMA_ARGS);
-    if (g == 5 && hw == 3 && q == 2) return launch_tma<5, 7, 2>(DEEDS_TMA_ARGS);
-    if (g == 4 && hw == 2 && q == 1) return launch_tma<4, 5, 1>(DEEDS_TMA_ARGS);
+#define DEEDS_MMA_ARGS d_F, d_Ms, m, n, o, len, q, pl, alpha1, d_cost, d_err, s
     switch (g) {
-        case 2: return launch_tma<2, 0, 0>(DEEDS_TMA_ARGS);
-        case 3: return launch_tma<3, 0, 0>(DEEDS_TMA_ARGS);
-        case 4: return launch_tma<4, 0, 0>(DEEDS_TMA_ARGS);
-        case 5: return launch_tma<5, 0, 0>(DEEDS_TMA_ARGS);
-        case 6: return launch_tma<6, 0, 0>(DEEDS_TMA_ARGS);
-        case 7: return launch_tma<7, 0, 0>(DEEDS_TMA_ARGS);
-        case 8: return launch_tma<8, 0, 0>(DEEDS_TMA_ARGS);
-        default: return cudaErrorInvalidValue;
+        case 2: return q == 1 ? launch_mma<2, true>(DEEDS_MMA_ARGS) : launch_mma<2, false>(DEEDS_MMA_ARGS);
+        case 3: return q == 1 ? launch_mma<3, true>(DEEDS_MMA_ARGS) : launch_mma<3, false>(DEEDS_MMA_ARGS);
+        case 4: return q == 1 ? launch_mma<4, true>(DEEDS_MMA_ARGS) : launch_mma<4, false>(DEEDS_MMA_ARGS);
+        case 5: return launch_mma<5, false>(DEEDS_MMA_ARGS);
+        case 6: return launch_mma<6, false>(DEEDS_MMA_ARGS);
+        case 7: return launch_mma<7, false>(DEEDS_MMA_ARGS);
+        default: return launch_mma<8, false>(DEEDS_MMA_ARGS);
     }
-#undef DEEDS_TMA_ARGS
+#undef DEEDS_MMA_ARGS
 }
 
 cudaError_t launch_data_cost(const uint64_t* d_F, const uint64_t* d_M, int m, int n, int o, int g, int hw, int q,
@@ -430,7 +684,7 @@ __global__ void k_selftest_mbar_wait(int* status) {
     if (threadIdx.x == 0) {
         mbar_init(&bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        *status = mbar_wait_bounded(&bar, 0) ? 2 : 1;
+        *status = mbar_wait(&bar, 0) ? 2 : 1;
     }
 }
 }  // namespace

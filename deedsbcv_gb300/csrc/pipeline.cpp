@@ -72,12 +72,6 @@ struct deeds_ctx {
     std::vector<Mark> marks;
     double stage_ms[DEEDS_NUM_STAGES] = {0};
     long long stage_launches[DEEDS_NUM_STAGES] = {0};
-    // cost-volume tile sizes chosen by the autotuner, per (g, hw, q); shared with batch lanes
-    struct TuneTable {
-        std::mutex mu;
-        std::map<std::vector<int>, int> tile;
-    };
-    std::shared_ptr<TuneTable> tune = std::make_shared<TuneTable>();
     // lanes of deeds_register_batch (child contexts on the same device)
     std::vector<deeds_ctx*> lanes;
     // the last registration's control-grid field (for deeds_warp_segmentation)
@@ -257,56 +251,15 @@ void data_cost_params(int g, int q, float alpha, int* sy, int* sx, int* sz, floa
     *alpha1 = (float)(0.5 * alphai / (float)maxsamp);
 }
 
-// Cost volume through the TMA-staged kernel when the shape allows it, with the
-// node-tile height chosen once per shape by timing the candidates (tiles only
-// change the schedule; every candidate writes the same bits).  Other shapes use
-// the generic kernel.
-cudaError_t data_cost_auto(deeds_ctx* ctx, const uint64_t* F, const uint64_t* M, uint64_t* Mpad, int m, int n, int o,
-                           int g, int hw, int q, float alpha, float* cost, int* d_err, cudaStream_t s) {
+// Cost volume on the tensor cores where the shape allows it, else by the generic kernel.
+cudaError_t data_cost_auto(const uint64_t* F, const uint64_t* M, uint64_t* split, int m, int n, int o, int g, int hw,
+                           int q, float alpha, float* cost, int* d_err, cudaStream_t s) {
     int sy, sx, sz;
     float alpha1;
     data_cost_params(g, q, alpha, &sy, &sx, &sz, &alpha1);
-    // the best tile depends on the level parameters, not on the volume size
-    const std::vector<int> key{g, hw, q};
-    std::lock_guard<std::mutex> lock(ctx->tune->mu);
-    auto it = ctx->tune->tile.find(key);
-    int tile;
-    if (it != ctx->tune->tile.end()) {
-        tile = it->second;
-    } else {
-        // tiles of whole warps' worth of (node, sample row) threads: 32k/g nodes
-        int cands[8];
-        for (int k = 1; k <= 8; k++) cands[k - 1] = 32 * k / g;
-        tile = 0;
-        float best = 1e30f;
-        cudaEvent_t a, b;
-        if (cudaEventCreate(&a) != cudaSuccess || cudaEventCreate(&b) != cudaSuccess) return cudaErrorUnknown;
-        // once per shape and context: time the candidates with the device otherwise
-        // idle (other streams of the registration would skew the comparison), best
-        // of three launches each after a warm-up launch
-        cudaDeviceSynchronize();
-        for (int c : cands) {
-            if (!data_cost_tma_supported(g, hw, q, c) || c > m / g) continue;
-            cudaError_t e = launch_data_cost_tma(F, M, Mpad, m, n, o, g, hw, q, c, alpha1, cost, d_err, s);
-            if (e != cudaSuccess) { cudaGetLastError(); continue; }
-            float c_best = 1e30f;
-            for (int r = 0; r < 3; r++) {
-                cudaEventRecord(a, s);
-                launch_data_cost_tma(F, M, Mpad, m, n, o, g, hw, q, c, alpha1, cost, d_err, s);
-                cudaEventRecord(b, s);
-                if (cudaEventSynchronize(b) != cudaSuccess) { cudaGetLastError(); break; }
-                float ms = 0.0f;
-                cudaEventElapsedTime(&ms, a, b);
-                c_best = std::min(c_best, ms);
-            }
-            if (c_best < best) { best = c_best; tile = c; }
-        }
-        cudaEventDestroy(a);
-        cudaEventDestroy(b);
-        ctx->tune->tile[key] = tile;
-    }
-    if (tile > m / g) tile = 0;  // tuned on a larger volume: this one has fewer grid rows
-    if (tile > 0) return launch_data_cost_tma(F, M, Mpad, m, n, o, g, hw, q, tile, alpha1, cost, d_err, s);
+    bool taken = false;
+    const cudaError_t e = launch_data_cost_mma(F, M, split, m, n, o, g, hw, q, alpha1, cost, d_err, s, &taken);
+    if (taken || e != cudaSuccess) return e;
     return launch_data_cost(F, M, m, n, o, g, hw, q, sy, sx, sz, alpha1, cost, s);
 }
 
@@ -442,7 +395,7 @@ deeds_status run_tree_bp(deeds_ctx* ctx, const std::string& tag, const PackedTre
 // Every buffer one registration of an m x n x o pair needs, sized up front so
 // that nothing is reallocated (cudaFree) while kernels of the pair are in flight.
 struct PairBuffers {
-    size_t max_sz1 = 0, max_cost = 0, max_pad = 0;
+    size_t max_sz1 = 0, max_cost = 0, max_split = 0;
     std::vector<int> m1s, n1s, o1s;
     float *fix, *mov, *warp0;
     // MIND codes of the fixed and of the affine-warped moving image, one pair per
@@ -455,7 +408,7 @@ struct PairBuffers {
     uint64_t* c_warp[2];
     float* mind_scr[2];
     float* cost[2];
-    uint64_t* mpad[2];
+    uint64_t* msplit[2];  // moving codes with their rows split by class (launch_data_cost_mma)
     float *grid, *kgrid, *cons_scr;  // kgrid: the last result's control-grid field (u | v | w)
     void* stats_scr;  // image statistics (deeds::launch_image_stats)
     float *d_stats, *h_stats;  // mean, std of the fixed and of the affine-warped moving image
@@ -475,7 +428,7 @@ deeds_status acquire_buffers(deeds_ctx* ctx, int m, int n, int o, const deeds_pa
         const size_t sz1 = (size_t)B.m1s[l] * B.n1s[l] * B.o1s[l];
         B.max_sz1 = std::max(B.max_sz1, sz1);
         B.max_cost = std::max(B.max_cost, sz1 * len * len * len);
-        B.max_pad = std::max(B.max_pad, padded_codes_count(m, n, o, P->quant[l] * P->radius[l]));
+        B.max_split = std::max(B.max_split, data_cost_split_count(m, n, o, P->grid[l], P->radius[l], P->quant[l]));
     }
     B.fix = dbuf<float>(ctx, "fix", sz, &st);
     B.mov = dbuf<float>(ctx, "mov", sz, &st);
@@ -500,7 +453,7 @@ deeds_status acquire_buffers(deeds_ctx* ctx, int m, int n, int o, const deeds_pa
         B.c_warp[d] = dbuf<uint64_t>(ctx, "c_warp_" + tg, sz, &st);
         B.mind_scr[d] = dbuf<float>(ctx, "mind_" + tg, 6 * sz, &st);
         B.cost[d] = dbuf<float>(ctx, "cost_" + tg, B.max_cost, &st);
-        B.mpad[d] = dbuf<uint64_t>(ctx, "mpad_" + tg, B.max_pad, &st);
+        B.msplit[d] = dbuf<uint64_t>(ctx, "msplit_" + tg, B.max_split, &st);
         dbuf<uint32_t>(ctx, "tree_" + tg, pack_layout((int)B.max_sz1).total, &st);
         dbuf<float>(ctx, "mins_" + tg, 4 * B.max_sz1, &st);
         dbuf<int>(ctx, "arrived_" + tg, B.max_sz1, &st);
@@ -665,16 +618,16 @@ deeds_status deeds_data_cost_dev(deeds_ctx* ctx, const uint64_t* d_F, const uint
         return fail(ctx, DEEDS_ERR_INVALID, "bad grid %d / radius %d / quant %d", g, hw, q);
     CK(cudaSetDevice(ctx->device));
     deeds_status st = DEEDS_OK;
-    uint64_t* mpad = dbuf<uint64_t>(ctx, "mpad_stage", padded_codes_count(m, n, o, q * hw), &st);
+    uint64_t* split = dbuf<uint64_t>(ctx, "msplit_stage", data_cost_split_count(m, n, o, g, hw, q), &st);
     int* d_err = dbuf<int>(ctx, "err_dc_stage", 1, &st);
     if (st) return st;
     cudaStream_t s = (cudaStream_t)stream;
     CK(cudaMemsetAsync(d_err, 0, sizeof(int), s));
-    CK(data_cost_auto(ctx, d_F, d_M, mpad, m, n, o, g, hw, q, alpha, d_cost, d_err, s));
+    CK(data_cost_auto(d_F, d_M, split, m, n, o, g, hw, q, alpha, d_cost, d_err, s));
     int herr = 0;
     CK(cudaMemcpyAsync(&herr, d_err, sizeof(int), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
-    if (herr) return fail(ctx, DEEDS_ERR_TIMEOUT, "cost volume: a bounded wait for a TMA copy expired");
+    if (herr) return fail(ctx, DEEDS_ERR_TIMEOUT, "cost volume: a bounded wait between its warps expired");
     return DEEDS_OK;
 }
 
@@ -857,7 +810,6 @@ deeds_status deeds_register_dev(deeds_ctx* ctx, const float* d_fixed, const floa
     uint64_t** c_warp = B.c_warp;
     float** mind_scr = B.mind_scr;
     float** cost = B.cost;
-    uint64_t** mpad = B.mpad;
     const char* tags[2] = {"f", "b"};
     float* grid = B.grid;
     float* cons_scr = B.cons_scr;
@@ -1014,7 +966,7 @@ deeds_status deeds_register_dev(deeds_ctx* ctx, const float* d_fixed, const floa
             // 192x160x256 pair, measured both ways).
             {
                 StageScope sc(ctx, DEEDS_STAGE_DATACOST, sdd);
-                CK(data_cost_auto(ctx, d == 0 ? c_fix : c_mov, reuse ? c_mov : c_warp[d], mpad[d], m, n, o, g, hw, q,
+                CK(data_cost_auto(d == 0 ? c_fix : c_mov, reuse ? c_mov : c_warp[d], B.msplit[d], m, n, o, g, hw, q,
                                   P->alpha, cost[d], d_err + d, sdd));
             }
             CK(cudaEventRecord(ctx->ev_cost[d], sdd));
@@ -1117,7 +1069,7 @@ deeds_status deeds_register_dev(deeds_ctx* ctx, const float* d_fixed, const floa
     if (builder.joinable()) builder.join();
     tl.dump();
     if (ctx->prof) collect_marks(ctx);
-    if (herr[0] == 3 || herr[1] == 3) return fail(ctx, DEEDS_ERR_TIMEOUT, "cost volume: a bounded wait for a TMA copy expired");
+    if (herr[0] == 3 || herr[1] == 3) return fail(ctx, DEEDS_ERR_TIMEOUT, "cost volume: a bounded wait between its warps expired");
     if (herr[0] == 4 || herr[1] == 4)
         return fail(ctx, DEEDS_ERR_TIMEOUT, "belief propagation: a bounded wait for a parent's label expired");
     if (herr[0] || herr[1])
@@ -1172,7 +1124,6 @@ deeds_status deeds_register_batch(deeds_ctx* ctx, const deeds_pair* pairs, int n
         deeds_ctx* lane = nullptr;
         deeds_status st = deeds_create(&lane, ctx->device);
         if (st) return fail(ctx, st, "batch lane: %s", deeds_last_error(nullptr));
-        lane->tune = ctx->tune;
         ctx->lanes.push_back(lane);
     }
     // size every lane's buffers for the largest pair up front: growing a buffer
@@ -1727,7 +1678,6 @@ deeds_status soft_lanes(deeds_ctx* ctx, int want) {
         deeds_ctx* lane = nullptr;
         deeds_status st = deeds_create(&lane, ctx->device);
         if (st) return fail(ctx, st, "batch lane: %s", deeds_last_error(nullptr));
-        lane->tune = ctx->tune;
         ctx->lanes.push_back(lane);
     }
     return DEEDS_OK;
@@ -2178,11 +2128,11 @@ deeds_status deeds_linear_register_dev(deeds_ctx* ctx, const float* d_fixed, con
     CK(cudaSetDevice(ctx->device));
     cudaStream_t s = (cudaStream_t)stream, sb = ctx->stream_b;
     const size_t sz = (size_t)m * n * o;
-    size_t max_cost = 0, max_pad = 0;
+    size_t max_cost = 0, max_split = 0;
     for (int l = 0; l < P->levels; l++) {
         const int g = P->grid[l], len = 2 * P->radius[l] + 1;
         max_cost = std::max(max_cost, (size_t)(m / g) * (n / g) * (o / g) * len * len * len);
-        max_pad = std::max(max_pad, padded_codes_count(m, n, o, P->quant[l] * P->radius[l]));
+        max_split = std::max(max_split, data_cost_split_count(m, n, o, P->grid[l], P->radius[l], P->quant[l]));
     }
     float* fix = dbuf<float>(ctx, "lin_fix", sz, &st);
     float* mov = dbuf<float>(ctx, "lin_mov", sz, &st);
@@ -2192,7 +2142,8 @@ deeds_status deeds_linear_register_dev(deeds_ctx* ctx, const float* d_fixed, con
     uint64_t* c_warp[2] = {dbuf<uint64_t>(ctx, "lin_c_w1", sz, &st), dbuf<uint64_t>(ctx, "lin_c_w2", sz, &st)};
     float* scr[2] = {dbuf<float>(ctx, "lin_mind1", 6 * sz, &st), dbuf<float>(ctx, "lin_mind2", 6 * sz, &st)};
     float* cost[2] = {dbuf<float>(ctx, "lin_cost1", max_cost, &st), dbuf<float>(ctx, "lin_cost2", max_cost, &st)};
-    uint64_t* mpad[2] = {dbuf<uint64_t>(ctx, "lin_mpad1", max_pad, &st), dbuf<uint64_t>(ctx, "lin_mpad2", max_pad, &st)};
+    uint64_t* msplit[2] = {dbuf<uint64_t>(ctx, "lin_msplit1", max_split, &st),
+                           dbuf<uint64_t>(ctx, "lin_msplit2", max_split, &st)};
     int* d_err = dbuf<int>(ctx, "lin_err", 2, &st);
     if (st) return st;
     float thr[5];
@@ -2232,7 +2183,7 @@ deeds_status deeds_linear_register_dev(deeds_ctx* ctx, const float* d_fixed, con
             }
             {
                 StageScope sc(ctx, DEEDS_STAGE_DATACOST, sd);
-                CK(data_cost_auto(ctx, d == 0 ? c_fix : c_mov, c_warp[d], mpad[d], m, n, o, g, hw, q, 1.0f, cost[d],
+                CK(data_cost_auto(d == 0 ? c_fix : c_mov, c_warp[d], msplit[d], m, n, o, g, hw, q, 1.0f, cost[d],
                                   d_err + d, sd));
             }
         }
@@ -2248,7 +2199,7 @@ deeds_status deeds_linear_register_dev(deeds_ctx* ctx, const float* d_fixed, con
     CK(cudaMemcpyAsync(herr, d_err, sizeof(herr), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     if (ctx->prof) collect_marks(ctx);
-    if (herr[0] == 3 || herr[1] == 3) return fail(ctx, DEEDS_ERR_TIMEOUT, "cost volume: a bounded wait for a TMA copy expired");
+    if (herr[0] == 3 || herr[1] == 3) return fail(ctx, DEEDS_ERR_TIMEOUT, "cost volume: a bounded wait between its warps expired");
     if (herr[0] || herr[1]) return fail(ctx, DEEDS_ERR_INTERNAL, "cost volume kernel reported error %d", herr[0] | herr[1]);
     std::memcpy(X_out, X, sizeof(X));
     return DEEDS_OK;
