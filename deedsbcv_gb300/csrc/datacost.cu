@@ -194,8 +194,9 @@ __global__ void __launch_bounds__(kCostThreads, 1)
     constexpr int S = G > 4 ? 2 : 1;  // x and z sampling stride (RAND_SAMPLES=1, src/dataCostD.h:141-155)
     constexpr int NX = (G + S - 1) / S, NZ = NX, NC = NX * NZ;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t b_full[4], b_done[4], b_acc[3], b_free[3], b_turn[2];
+    __shared__ __align__(8) uint64_t b_full[4], b_done[8], b_acc[3], b_free[3], b_turn[2];
     __shared__ uint32_t s_tmem;
+    __shared__ int s_failed;
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int len2 = len * len, len3 = len2 * len;
@@ -215,7 +216,8 @@ __global__ void __launch_bounds__(kCostThreads, 1)
     const int n_groups = min(pl.groups_per_cta, pl.groups - g_first);
     const int ly0 = blockIdx.z * pl.nly;
     const int n_ly = min(pl.nly, len - ly0);
-    const int group_tiles = q * len, n_tiles = n_groups * group_tiles;
+    const int group_tiles = q * len;
+    int n_tiles = n_groups * group_tiles, n_steps = n_groups * len;
     const int y_first = ty * pl.tn, y0 = y_first * G;
     const int pad = q * (len - 1) / 2;
     const int y0_q = y0 / q, y0_res = y0 - y0_q * q;
@@ -224,10 +226,8 @@ __global__ void __launch_bounds__(kCostThreads, 1)
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&s_tmem))
                      : "memory");
         if (lane == 0) {
-            for (int i = 0; i < 4; i++) {
-                mbar_init(&b_full[i], 4);
-                mbar_init(&b_done[i], 1);
-            }
+            for (int i = 0; i < 4; i++) mbar_init(&b_full[i], 4);
+            for (int i = 0; i < 8; i++) mbar_init(&b_done[i], 1);
             for (int i = 0; i < kEpiGroups; i++) {
                 mbar_init(&b_acc[i], 1);
                 mbar_init(&b_free[i], 4);
@@ -236,11 +236,13 @@ __global__ void __launch_bounds__(kCostThreads, 1)
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
     }
+    if (tid == 0) s_failed = *(volatile int*)err;  // a wait of an earlier CTA gave up: no further waits
     for (int e = tid; e < pl.tn; e += kCostThreads) s_term[e] = 0;
     tmem_fence_before();
     __syncthreads();
     tmem_fence_after();
     const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
+    if (s_failed) n_tiles = n_steps = 0;
     if (warp < 4) {  // unit scales (E8M0 127) in every byte of the scale columns
         const uint32_t one = 0x7f7f7f7fu;
         const uint32_t w[8] = {one, one, one, one, one, one, one, one};
@@ -270,7 +272,7 @@ __global__ void __launch_bounds__(kCostThreads, 1)
     __syncthreads();
     tmem_fence_after();
 
-    const auto wait_done = [&](int t) { return mbar_wait(&b_done[t & 3], (uint32_t)((t >> 2) & 1)); };
+    const auto wait_done = [&](int t) { return mbar_wait(&b_done[t & 7], (uint32_t)((t >> 3) & 1)); };
     const auto wait_full = [&](int t) { return mbar_wait(&b_full[t & 3], (uint32_t)((t >> 2) & 1)); };
     const uint32_t quadrant = (uint32_t)((warp & 3) * 32) << 16;
     const int row = tid & 127;
@@ -315,8 +317,10 @@ __global__ void __launch_bounds__(kCostThreads, 1)
         if (wg < n_tiles) load();
         for (int t = wg; t < n_tiles; t += kProdGroups) {
             // the columns overwritten were last read by tile t - 3 or before: a tile
-            // moves the ring by at most NX <= 4 of its 12 columns.  (Every tile's phase is
-            // waited for in turn: a parity says nothing about the phase before it.)
+            // moves the ring by at most NX <= 4 of its 12 columns.  (A parity tells a phase
+            // only from its neighbours: every tile's phase is waited for in turn, so the one
+            // before it is over, and the next use of a barrier is tile t + 3 or later, which
+            // cannot be issued before this tile is in place, so none is missed.)
             for (int d = kProdGroups + 2; d >= 3 && ok; d--)
                 if (t >= d) ok = wait_done(t - d);
             ok = __all_sync(0xffffffffu, ok);
@@ -360,7 +364,6 @@ __global__ void __launch_bounds__(kCostThreads, 1)
 #pragma unroll
         for (int i = 0; i < kSums; i++) sum_of(row + i * 128, s_at[i], s_out[i], s_k[i]);
         float* const cost0 = cost + (int64_t)(y_first + nxn * m1 + nzn * m1 * n1) * len3 + ly0;
-        const int n_steps = n_groups * len;
         int lx = e, gi = 0;
         while (lx >= len) { lx -= len; gi++; }
         for (int st = e; st < n_steps; st += kEpiGroups) {
@@ -418,7 +421,6 @@ __global__ void __launch_bounds__(kCostThreads, 1)
         const uint32_t blo0 = ((smem_u32(smem_raw) & 0x3ffffu) >> 4) | ((uint32_t)pl.N << 16);
         const uint32_t bhi = 8u | (1u << 14), sf = tmem + kColS;
         int last = -1;  // the last step committed
-        const int n_steps = n_groups * len;
         int x = 0, col = 0;  // the step's number in its group, its first ring column
         const auto next = [&]() {
             col += q * USTEP;
@@ -457,7 +459,7 @@ __global__ void __launch_bounds__(kCostThreads, 1)
                             else mma_mxf4<false>(d, a + k * 8, bl, bhi, idesc, sf, sf + 8, 1u);
                         }
                     }
-                    mma_commit(&b_done[t & 3]);
+                    mma_commit(&b_done[t & 7]);
                     if (r == q - 1) mma_commit(&b_acc[acc]);
                 }
                 __syncwarp();
@@ -520,6 +522,7 @@ __global__ void __launch_bounds__(256) k_data_cost(const uint64_t* __restrict__ 
     }
 }
 
+constexpr int kMaxSmem = 200 * 1024;
 size_t cost_smem(const CostPlan& c, int g, int q) {
     const int S = g > 4 ? 2 : 1, NX = (g + S - 1) / S;
     return (size_t)q * NX * NX * c.N * 32 + (size_t)epi_groups(q == 1 && g <= 4) * c.N * kEntryPitch * 4 + (size_t)c.tn * 4;
@@ -555,7 +558,7 @@ bool cost_plan(int m, int n, int o, int g, int len, int q, CostPlan& best) {
         for (c.P = 1; c.P * c.R <= 128 && c.P <= len; c.P++) {
             c.groups = (len + c.P - 1) / c.P;
             if (c.P > 1 && c.groups == (len + c.P - 2) / (c.P - 1)) continue;
-            if (cost_smem(c, g, q) > 200 * 1024) continue;
+            if (cost_smem(c, g, q) > kMaxSmem) continue;
             const bool slide = q == 1 && g <= 4;
             const double rounds = (c.P * tn * nly + 127) / 128;
             const double mma = slide ? NC * 22.0 + 350.0 : q * (NC * 33.0 + 320.0);
@@ -585,7 +588,8 @@ template <int G, bool SLIDE>
 cudaError_t launch_mma(const uint64_t* d_F, const uint64_t* d_Ms, int m, int n, int o, int len, int q,
                        const CostPlan& pl, float alpha1, float* d_cost, int* d_err, cudaStream_t s) {
     const size_t smem = cost_smem(pl, G, q);
-    cudaError_t e = cudaFuncSetAttribute(k_data_cost_mma<G, SLIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the same limit on every call: other threads launch the kernel for other sizes
+    cudaError_t e = cudaFuncSetAttribute(k_data_cost_mma<G, SLIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
     if (e != cudaSuccess) return e;
     const dim3 grid((unsigned)(pl.tiles_y * (n / G) * (o / G)), (unsigned)pl.splits, (unsigned)pl.chunks);
     k_data_cost_mma<G, SLIDE><<<grid, kCostThreads, smem, s>>>(d_F, d_Ms, d_cost, m, n, o, len, q, pl, alpha1, d_err);
@@ -632,7 +636,8 @@ cudaError_t launch_data_cost(const uint64_t* d_F, const uint64_t* d_M, int m, in
     const int ns = ((g + sy - 1) / sy) * ((g + sx - 1) / sx) * ((g + sz - 1) / sz);
     const size_t smem = (size_t)ns * sizeof(uint64_t);
     if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k_data_cost, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(k_data_cost, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             std::max(kMaxSmem, (int)smem));  // as above: one limit for all
         if (e != cudaSuccess) return e;
     }
     const int len3 = (2 * hw + 1) * (2 * hw + 1) * (2 * hw + 1);
