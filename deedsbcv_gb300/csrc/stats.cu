@@ -20,16 +20,18 @@
 // and its shifted copy stay inside the binade, and evaluates every other segment
 // from the true start.  The result is the reference's to the bit for any data.
 //
-// Two levels: chunks of 2048 elements; a chunk whose own trajectory leaves its
+// Two levels: chunks of 512 elements; a chunk whose own trajectory leaves its
 // binade or comes near one of its ends (the sum crosses a power of two: about
 // log2(sum / first element) chunks per chain) or that has no usable estimate is
 // also run as 32 sub-segments, in parallel before the walk, so the walk replays
-// at most a few sub-segments of 65 elements (staged in shared memory) where a
+// at most a few sub-segments of 17 elements (staged in shared memory) where a
 // chunk fails.  No thread walks a long stretch of global memory alone.
 //
-// Work: 4 B per voxel read by the chunk sums and once per chain, plus the
-// crossing chunks twice more.  Dependency bound: 2048 steps per chunk chain and
-// ~4000 sequential chunk checks (bit operations and float compares).
+// Work: 4 B per voxel read by the chunk sums and twice per chain, plus the crossing
+// chunks twice more.  Dependency bound: 512 steps per chunk trajectory, four passes of
+// them, and two walks (32 chunks at a time by composing their maps; ~15 crossing
+// chunks each, one sub-segment after the other).  One image of 192x160x256: 2.96 -> 0.95 ms
+// (chunks of 2048 walked one by one, estimates in one block); of 56x48x64 0.6 ms.
 #include <algorithm>
 #include <cmath>
 
@@ -40,7 +42,7 @@ namespace deeds {
 
 namespace {
 
-constexpr int kStatsChunk = 2048;  // elements per chunk (bounds sz * c / nch: 2048 to 4095)
+constexpr int kStatsChunk = 512;  // elements per chunk (bounds sz * c / nch: 512 to 1023)
 constexpr int kSub = 32;           // sub-segments of a chunk run in parallel
 
 struct ChunkRun {
@@ -219,97 +221,159 @@ __device__ __forceinline__ void stage_async(float* dst, const float* __restrict_
     __syncwarp();
 }
 
-// Chunk sums in double (estimates of the chains' values at chunk starts; any
-// order of addition).  Grid (nch, nimg), 256 threads.
+// Chunk sums (estimates of the chains' values at chunk starts; any order of addition):
+// one warp per chunk, the lanes' 16 to 32 elements added in float about the lane's
+// first one (FP64 adds of every element were the bound: 0.18 ms at 192x160x256), the
+// lanes' sums in double.  Grid (ceil(nch / 8), nimg), 256 threads.
 __global__ void __launch_bounds__(256) k_stats_sums(const float* __restrict__ im0, const float* __restrict__ im1,
                                                     size_t sz, int nch, double* __restrict__ sx,
                                                     double* __restrict__ sx2) {
     const float* x = blockIdx.y == 0 ? im0 : im1;
-    const int c = blockIdx.x;
-    const size_t lo = chunk_lo(sz, nch, c), hi = chunk_lo(sz, nch, c + 1);
-    double s = 0.0, q = 0.0;
-    for (size_t i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-        const double v = x[i];
-        s += v;
-        q += v * v;
+    const int c = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (c >= nch) return;
+    const size_t lo = chunk_lo(sz, nch, c);
+    const int n = (int)(chunk_lo(sz, nch, c + 1) - lo);
+    const float x0 = lane < n ? __ldg(x + lo + lane) : 0.0f;
+    float a = 0.0f, b = 0.0f;  // sums of x - x0 and of its square
+    int cnt = 0;
+    for (int i = lane; i < n; i += 32, cnt++) {
+        const float d = __ldg(x + lo + i) - x0;
+        a += d;
+        b += d * d;
     }
-    __shared__ double red_s[8], red_q[8];
+    const double dx0 = x0, da = a;
+    double s = cnt * dx0 + da;
+    double q = (double)b + 2.0 * dx0 * da + cnt * dx0 * dx0;
     for (int o = 16; o > 0; o >>= 1) {
         s += __shfl_xor_sync(0xffffffffu, s, o);
         q += __shfl_xor_sync(0xffffffffu, q, o);
     }
-    const int w = threadIdx.x >> 5;
-    if ((threadIdx.x & 31) == 0) {
-        red_s[w] = s;
-        red_q[w] = q;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double ts = 0.0, tq = 0.0;
-        for (int k = 0; k < (int)(blockDim.x >> 5); k++) {
-            ts += red_s[k];
-            tq += red_q[k];
-        }
-        sx[(size_t)blockIdx.y * nch + c] = ts;
-        sx2[(size_t)blockIdx.y * nch + c] = tq;
+    if (lane == 0) {
+        sx[(size_t)blockIdx.y * nch + c] = s;
+        sx2[(size_t)blockIdx.y * nch + c] = q;
     }
 }
 
-// Start estimates of every chunk (exclusive prefix of the chunk sums; for the
-// variance, sum (x - m)^2 = sum x^2 - 2 m sum x + n m^2 with the estimated mean
-// m) and the two starts of each chunk's trajectories.  One block of 1024 threads
-// per image; each thread scans a run of consecutive chunks.
-template <int KIND>
+// Exclusive prefix of a over the block's 1024 threads, and the block's total.
+__device__ __forceinline__ double block_scan(double a, double* warp_sum, double& total) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    double incl = a;
+    for (int o = 1; o < 32; o <<= 1) {
+        const double y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    __syncthreads();  // the previous call's readers are done
+    if (lane == 31) warp_sum[w] = incl;
+    __syncthreads();
+    double ws = warp_sum[lane];
+    for (int o = 1; o < 32; o <<= 1) {
+        const double y = __shfl_up_sync(0xffffffffu, ws, o);
+        if (lane >= o) ws += y;
+    }
+    total = __shfl_sync(0xffffffffu, ws, 31);
+    const double before = __shfl_sync(0xffffffffu, ws, w > 0 ? w - 1 : 0);
+    return (w > 0 ? before : 0.0) + incl - a;
+}
+
+// Start estimates of every chunk, and the two starts of its trajectories: the exclusive
+// prefix of an increment per chunk.  AGAIN false: the chunk sums; for the variance,
+// sum (x - m)^2 = sum x^2 - 2 m sum x + n m^2 with the estimated mean m.  AGAIN true:
+// the first pass's float increments (end - start of each speculated chunk's trajectory;
+// the chunk sum where there was none).  The float chain drops the parts of small terms
+// that round away against a large sum, so these follow the true chain far more closely
+// than the exact sums do.  A block of 1024 threads takes 1024 chunks and adds up all
+// increments before them itself (FP64 is slow: one block for all chunks took 0.12 ms).
+// Grid (ceil(nch / 1024), nimg).
+template <int KIND, bool AGAIN>
 __global__ void __launch_bounds__(1024) k_stats_starts(size_t sz, int nch, const double* __restrict__ sx,
-                                                       const double* __restrict__ sx2, ChunkRun* __restrict__ run) {
-    const int img = blockIdx.x;
+                                                       const double* __restrict__ sx2, double* __restrict__ inc,
+                                                       ChunkRun* __restrict__ run) {
+    const int img = blockIdx.y;
     const double* s = sx + (size_t)img * nch;
     const double* q = sx2 + (size_t)img * nch;
-    ChunkRun* r = run + (size_t)img * nch;
-    __shared__ double part[1024];
-    __shared__ double total_s;
-    const int T = blockDim.x, t = threadIdx.x;
-    const int per = (nch + T - 1) / T;
-    const int c0 = min(nch, t * per), c1 = min(nch, c0 + per);
-    double m = 0.0;
-    if (KIND == 1) {
+    inc += (size_t)img * nch;
+    __shared__ double warp_sum[32];
+    double m = 0.0, nmm = 0.0, total;
+    if (KIND == 1 && !AGAIN) {
         double a = 0.0;
-        for (int c = c0; c < c1; c++) a += s[c];
-        part[t] = a;
-        __syncthreads();
-        if (t == 0) {
-            double tot = 0.0;
-            for (int k = 0; k < T; k++) tot += part[k];
-            total_s = tot;
-        }
-        __syncthreads();
-        m = total_s / (double)sz;
-        __syncthreads();
+        for (int c = threadIdx.x; c < nch; c += 1024) a += s[c];
+        block_scan(a, warp_sum, total);
+        m = total / (double)sz;
+        nmm = (double)sz / nch * m * m;  // n m^2 of a chunk of mean length
     }
-    auto term = [&](int c) {
+    auto increment = [&](int c) {
+        if (AGAIN) return inc[c];
         if (KIND == 0) return s[c];
-        const double n = (double)(chunk_lo(sz, nch, c + 1) - chunk_lo(sz, nch, c));
-        return fmax(0.0, q[c] - 2.0 * m * s[c] + n * m * m);
+        return fmax(0.0, q[c] - 2.0 * m * s[c] + nmm);
     };
-    double a = 0.0;
-    for (int c = c0; c < c1; c++) a += term(c);
-    part[t] = a;
-    __syncthreads();
-    // inclusive Hillis-Steele scan of the per-thread totals
-    for (int off = 1; off < T; off <<= 1) {
-        const double v = t >= off ? part[t - off] : 0.0;
-        __syncthreads();
-        part[t] += v;
-        __syncthreads();
-    }
-    double pre = t > 0 ? part[t - 1] : 0.0;
-    for (int c = c0; c < c1; c++) {
-        const float est = (float)pre;
-        pre += term(c);
+    const int c0 = blockIdx.x * 1024, c = c0 + threadIdx.x;
+    double before = 0.0, pre;
+    for (int k = threadIdx.x; k < c0; k += 1024) before += increment(k);
+    block_scan(before, warp_sum, pre);
+    const double mine = c < nch ? increment(c) : 0.0;
+    const float est = (float)(pre + block_scan(mine, warp_sum, total));
+    if (c < nch) {
         ChunkRun cr;
         spec_starts(est, cr);
-        r[c] = cr;
+        run[(size_t)img * nch + c] = cr;
+        if (!AGAIN) inc[c] = mine;
     }
+}
+
+// What a run of chunks does to an integer value V of either parity q: V + delta[q] after
+// it, its values between V + lo[q] and V + hi[q] (lo > hi: not known).
+struct Step {
+    int delta[2], lo[2], hi[2];
+};
+// All entries saturate at +-kNever, far outside any binade (2^24 units): delta, the last
+// of the values between lo and hi, only where lo or hi does, so a map that would need
+// more than that is refused.
+constexpr int kNever = 1 << 29;
+__device__ __forceinline__ int saturate(int x) { return max(-kNever, min(kNever, x)); }
+
+// `f`, then the step held by the lane `off` above.
+__device__ __forceinline__ Step then_lane(const Step& f, int off) {
+    Step g, r;
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        g.delta[q] = __shfl_down_sync(0xffffffffu, f.delta[q], off);
+        g.lo[q] = __shfl_down_sync(0xffffffffu, f.lo[q], off);
+        g.hi[q] = __shfl_down_sync(0xffffffffu, f.hi[q], off);
+    }
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        const bool odd = ((q ^ f.delta[q]) & 1) != 0;
+        r.delta[q] = saturate(f.delta[q] + (odd ? g.delta[1] : g.delta[0]));
+        r.lo[q] = saturate(min(f.lo[q], f.delta[q] + (odd ? g.lo[1] : g.lo[0])));
+        r.hi[q] = saturate(max(f.hi[q], f.delta[q] + (odd ? g.hi[1] : g.hi[0])));
+    }
+    return r;
+}
+
+// The composed map of the lanes' steps, in lane order (lane 0 holds it).
+__device__ __forceinline__ Step compose_lanes(Step f) {
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) f = then_lane(f, off);
+    return f;
+}
+
+// 32 consecutive chunks' composed map in the binade e of sign neg; e = 0: not all of
+// them have one.
+struct BatchRec {
+    int e, neg;
+    Step f;
+};
+
+// V through the map f, if every value on the way stays inside the binade
+__device__ __forceinline__ bool apply_step(const Step& f, int neg, int& V) {
+    constexpr int IN = (1 << 23) + 1, OUT = (1 << 24) - 2;
+    const int q = V & 1;
+    const int lo = q ? f.lo[1] : f.lo[0], hi = q ? f.hi[1] : f.hi[0];
+    if (lo <= -kNever / 2 || hi >= kNever / 2) return false;
+    const int l = V + lo, h = V + hi;
+    if (!(neg ? (l >= -OUT && h <= -IN) : (l >= IN && h <= OUT))) return false;
+    V += q ? f.delta[1] : f.delta[0];
+    return true;
 }
 
 // Both trajectories of every speculated chunk, one lane per chunk: a warp owns
@@ -318,11 +382,12 @@ __global__ void __launch_bounds__(1024) k_stats_starts(size_t sz, int nch, const
 // a padded shared tile that each lane then reads along its own row.  A chunk
 // whose trajectory leaves its binade or comes near one of its ends, or that has
 // no usable estimate, is marked for sub-segment runs; every chunk's integer
-// walk record is written.  Grid (ceil(nch / 32), nimg), 32 threads.
+// walk record and the 32 chunks' composed map are written.  Grid (ceil(nch / 32), nimg), 32 threads.
 template <int KIND>
 __global__ void __launch_bounds__(32) k_stats_traj(const float* __restrict__ im0, const float* __restrict__ im1,
                                                    size_t sz, int nch, const float* __restrict__ means,
-                                                   ChunkRun* __restrict__ run, WalkRec* __restrict__ walk) {
+                                                   double* __restrict__ inc, ChunkRun* __restrict__ run,
+                                                   WalkRec* __restrict__ walk, BatchRec* __restrict__ batches) {
     __shared__ float tile[32][33];
     const float* x = blockIdx.y == 0 ? im0 : im1;
     const int lane = threadIdx.x;
@@ -352,15 +417,13 @@ __global__ void __launch_bounds__(32) k_stats_traj(const float* __restrict__ im0
         }
         __syncwarp();
     }
-    if (c >= nch) return;
     // also marked: chunks whose trajectory comes within 2^-12 of the binade's
     // width of an end, which a shift onto the true start could push out
     int e = 0;
     float u = 0.0f;
     bool in = cr.spec && binade(cr.start_a, e, u);
     const bool neg = signbit(cr.start_a);
-    WalkRec w;
-    w.e = 0;
+    WalkRec w = {};
     if (in) {
         const float margin = pow2f(e - 13);
         // (fminf / fmaxf skip NaN, so a trajectory that met a NaN is recognised by its end)
@@ -381,68 +444,28 @@ __global__ void __launch_bounds__(32) k_stats_traj(const float* __restrict__ im0
     }
     cr.cross = !in;
     w.cross = cr.cross;
-    run[(size_t)blockIdx.y * nch + c] = cr;
-    walk[(size_t)blockIdx.y * nch + c] = w;
-}
-
-// Second estimates of every chunk's start: the exclusive prefix of the first
-// pass's float increments (end - start of each speculated chunk's trajectory;
-// the double chunk sum where there was none).  The float chain drops the parts
-// of small terms that round away against a large sum, so these follow the true
-// chain far more closely than the exact sums do.  One block of 1024 threads per
-// image.
-template <int KIND>
-__global__ void __launch_bounds__(1024) k_stats_restarts(size_t sz, int nch, const double* __restrict__ sx,
-                                                         const double* __restrict__ sx2, ChunkRun* __restrict__ run) {
-    const int img = blockIdx.x;
-    const double* s = sx + (size_t)img * nch;
-    const double* q = sx2 + (size_t)img * nch;
-    ChunkRun* r = run + (size_t)img * nch;
-    __shared__ double part[1024];
-    __shared__ double total_s;
-    const int T = blockDim.x, t = threadIdx.x;
-    const int per = (nch + T - 1) / T;
-    const int c0 = min(nch, t * per), c1 = min(nch, c0 + per);
-    double m = 0.0;
-    if (KIND == 1) {
-        double a = 0.0;
-        for (int c = c0; c < c1; c++) a += s[c];
-        part[t] = a;
-        __syncthreads();
-        if (t == 0) {
-            double tot = 0.0;
-            for (int k = 0; k < T; k++) tot += part[k];
-            total_s = tot;
-        }
-        __syncthreads();
-        m = total_s / (double)sz;
-        __syncthreads();
+    if (c < nch) {
+        run[(size_t)blockIdx.y * nch + c] = cr;
+        walk[(size_t)blockIdx.y * nch + c] = w;
+        if (cr.spec) inc[(size_t)blockIdx.y * nch + c] = (double)cr.end_a - (double)cr.start_a;
     }
-    auto inc = [&](int c) {
-        const ChunkRun& cr = r[c];
-        if (cr.spec) return (double)cr.end_a - (double)cr.start_a;
-        if (KIND == 0) return s[c];
-        const double n = (double)(chunk_lo(sz, nch, c + 1) - chunk_lo(sz, nch, c));
-        return fmax(0.0, q[c] - 2.0 * m * s[c] + n * m * m);
-    };
-    double a = 0.0;
-    for (int c = c0; c < c1; c++) a += inc(c);
-    part[t] = a;
-    __syncthreads();
-    for (int off = 1; off < T; off <<= 1) {
-        const double v = t >= off ? part[t - off] : 0.0;
-        __syncthreads();
-        part[t] += v;
-        __syncthreads();
+    // the 32 chunks' composed map
+    BatchRec br;
+    br.e = __shfl_sync(0xffffffffu, w.e, 0);
+    br.neg = __shfl_sync(0xffffffffu, w.neg, 0);
+    Step f;
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        const bool a = (w.sa & 1) == q;
+        const int S = a ? w.sa : w.sb, LO = a ? w.loa : w.lob, HI = a ? w.hia : w.hib;
+        const bool ok = c < nch && LO <= HI;
+        f.delta[q] = ok ? (a ? w.ea : w.eb) - S : 0;
+        f.lo[q] = c >= nch ? 0 : ok ? LO - S : -kNever;
+        f.hi[q] = c >= nch ? 0 : ok ? HI - S : kNever;
     }
-    double pre = t > 0 ? part[t - 1] : 0.0;
-    for (int c = c0; c < c1; c++) {  // each thread rewrites only its own chunks
-        const float est = (float)pre;
-        pre += inc(c);
-        ChunkRun cr;
-        spec_starts(est, cr);
-        r[c] = cr;
-    }
+    if (!__all_sync(0xffffffffu, c >= nch || (w.e == br.e && w.neg == br.neg))) br.e = 0;
+    br.f = compose_lanes(f);
+    if (lane == 0) batches[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = br;
 }
 
 // Sub-segment runs of the chunks marked by k_stats_traj: the chunk is staged in
@@ -540,56 +563,86 @@ __device__ float warp_segment(const float* __restrict__ xg, int n, float v, floa
 // of u, and a chunk whose trajectory (chosen by the parity of V - its start) and
 // that trajectory shifted by V - start stay inside the binade gives V' = its end
 // + the shift, with integer operations only; any other chunk is evaluated by
-// warp_segment from the float value.  The walk records are read 32 at a time.
+// warp_segment from the float value.  Chunks are taken 1024 at a time where they all
+// qualify (the lanes compose the maps of their 32 chunks), else 32 at a time, else one
+// by one.
 // KIND 0 writes the mean, KIND 1 the standard deviation (out[2 img + 0 / 1]).
 // Dynamic shared memory: the largest chunk.
 template <int KIND>
 __global__ void __launch_bounds__(32) k_stats_stitch(const float* __restrict__ im0, const float* __restrict__ im1,
                                                      size_t sz, int nch, const ChunkRun* __restrict__ run,
-                                                     const WalkRec* __restrict__ walk, const ChunkRun* __restrict__ sub,
-                                                     float* __restrict__ means, float* __restrict__ out) {
+                                                     const WalkRec* __restrict__ walk,
+                                                     const BatchRec* __restrict__ batches,
+                                                     const ChunkRun* __restrict__ sub, float* __restrict__ means,
+                                                     float* __restrict__ out) {
     extern __shared__ float buf[];
     __shared__ WalkRec batch[32];
+    __shared__ BatchRec group[32];
     const int img = blockIdx.x, lane = threadIdx.x;
     const float* x = img == 0 ? im0 : im1;
     const float mean = KIND == 1 ? means[img] : 0.0f;
     constexpr int IN = (1 << 23) + 1, OUT = (1 << 24) - 2;
+    const int nbatch = (nch + 31) / 32;
     float v = 0.0f;
     int ve = 0, vneg = 0, V = 0;  // ve = 0: v is not held as an integer (0, tiny or not finite)
-    // the next batch of records is loaded into registers while this one is walked
-    WalkRec nextrec;
-    if (lane < nch) nextrec = walk[(size_t)img * nch + lane];
-    for (int c0 = 0; c0 < nch && !isnan(v); c0 += 32) {
+    // the next group of maps is loaded into registers while this one is walked
+    BatchRec nextrec = {};
+    if (lane < nbatch) nextrec = batches[(size_t)img * nbatch + lane];
+    for (int b0 = 0; b0 < nbatch && !isnan(v); b0 += 32) {
+        const BatchRec mine = nextrec;
         __syncwarp();
-        batch[lane] = nextrec;
-        if (c0 + 32 + lane < nch) nextrec = walk[(size_t)img * nch + c0 + 32 + lane];
+        group[lane] = mine;
+        nextrec = BatchRec{};
+        if (b0 + 32 + lane < nbatch) nextrec = batches[(size_t)img * nbatch + b0 + 32 + lane];
         __syncwarp();
-        const int nb = min(32, nch - c0);
-        for (int k = 0; k < nb; k++) {
-            const WalkRec& w = batch[k];
-            bool ok = false;
-            if (ve != 0 && w.e == ve && w.neg == vneg) {
-                const bool odd = ((V - w.sa) & 1) != 0;
-                const int S = odd ? w.sb : w.sa, E = odd ? w.eb : w.ea;
-                const int LO = odd ? w.lob : w.loa, HI = odd ? w.hib : w.hia;
-                const int D = V - S, l = LO + D, h = HI + D;
-                ok = LO <= HI && (vneg ? (l >= -OUT && h <= -IN) : (l >= IN && h <= OUT));
-                if (ok) V = E + D;
+        const int ng = min(32, nbatch - b0);
+        if (ve != 0 && __all_sync(0xffffffffu, lane >= ng || (mine.e == ve && mine.neg == vneg))) {
+            Step f = mine.f;
+            if (lane >= ng) f = Step{};
+            f = compose_lanes(f);
+            Step whole;
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                whole.delta[q] = __shfl_sync(0xffffffffu, f.delta[q], 0);
+                whole.lo[q] = __shfl_sync(0xffffffffu, f.lo[q], 0);
+                whole.hi[q] = __shfl_sync(0xffffffffu, f.hi[q], 0);
             }
-            if (ok) continue;
-            // the float value, then the chunk exactly
-            if (ve != 0) v = (float)V * pow2f(ve - 24);
-            if (isnan(v)) break;  // absorbing for both chains: the result is NaN
-            const int c = c0 + k;
-            const size_t lo = chunk_lo(sz, nch, c), hi = chunk_lo(sz, nch, c + 1);
-            const ChunkRun* sr = w.cross ? sub + ((size_t)img * nch + c) * kSub : nullptr;
-            v = warp_segment<KIND>(x + lo, (int)(hi - lo), v, mean, sr, buf);
-            float u;
-            if (binade(v, ve, u)) {
-                vneg = signbit(v) ? 1 : 0;
-                V = (int)(v * pow2f(24 - ve));
-            } else {
-                ve = 0;
+            if (apply_step(whole, vneg, V)) continue;
+        }
+        for (int g = 0; g < ng && !isnan(v); g++) {
+            const BatchRec& br = group[g];
+            if (ve != 0 && br.e == ve && br.neg == vneg && apply_step(br.f, vneg, V)) continue;
+            const int c0 = (b0 + g) * 32;
+            __syncwarp();
+            if (c0 + lane < nch) batch[lane] = walk[(size_t)img * nch + c0 + lane];
+            __syncwarp();
+            const int nb = min(32, nch - c0);
+            for (int k = 0; k < nb; k++) {
+                const WalkRec& w = batch[k];
+                bool ok = false;
+                if (ve != 0 && w.e == ve && w.neg == vneg) {
+                    const bool odd = ((V - w.sa) & 1) != 0;
+                    const int S = odd ? w.sb : w.sa, E = odd ? w.eb : w.ea;
+                    const int LO = odd ? w.lob : w.loa, HI = odd ? w.hib : w.hia;
+                    const int D = V - S, l = LO + D, h = HI + D;
+                    ok = LO <= HI && (vneg ? (l >= -OUT && h <= -IN) : (l >= IN && h <= OUT));
+                    if (ok) V = E + D;
+                }
+                if (ok) continue;
+                // the float value, then the chunk exactly
+                if (ve != 0) v = (float)V * pow2f(ve - 24);
+                if (isnan(v)) break;  // absorbing for both chains: the result is NaN
+                const int c = c0 + k;
+                const size_t lo = chunk_lo(sz, nch, c), hi = chunk_lo(sz, nch, c + 1);
+                const ChunkRun* sr = w.cross ? sub + ((size_t)img * nch + c) * kSub : nullptr;
+                v = warp_segment<KIND>(x + lo, (int)(hi - lo), v, mean, sr, buf);
+                float u;
+                if (binade(v, ve, u)) {
+                    vneg = signbit(v) ? 1 : 0;
+                    V = (int)(v * pow2f(24 - ve));
+                } else {
+                    ve = 0;
+                }
             }
         }
     }
@@ -614,7 +667,8 @@ constexpr int kSegSmemMax = (int)((2 * (size_t)kStatsChunk + 2) * sizeof(float))
 
 size_t image_stats_scratch_bytes(size_t sz, int nimg) {
     const size_t nch = (size_t)stats_chunks(sz);
-    return 256 + (size_t)nimg * nch * (2 * sizeof(double) + sizeof(ChunkRun) * (1 + kSub) + sizeof(WalkRec)) + 64;
+    return 256 + (size_t)nimg * nch * (3 * sizeof(double) + sizeof(ChunkRun) * (1 + kSub) + sizeof(WalkRec)) +
+           (size_t)nimg * ((nch + 31) / 32) * sizeof(BatchRec) + 64;
 }
 
 // Mean and standard deviation of one or two images (im1 may be null when nimg
@@ -631,11 +685,15 @@ cudaError_t launch_image_stats(const float* im0, const float* im1, int nimg, siz
     p += (size_t)nimg * nch * sizeof(double);
     double* sx2 = reinterpret_cast<double*>(p);
     p += (size_t)nimg * nch * sizeof(double);
+    double* inc = reinterpret_cast<double*>(p);
+    p += (size_t)nimg * nch * sizeof(double);
     ChunkRun* run = reinterpret_cast<ChunkRun*>(p);
     p += (size_t)nimg * nch * sizeof(ChunkRun);
     ChunkRun* sub = reinterpret_cast<ChunkRun*>(p);
     p += (size_t)nimg * nch * kSub * sizeof(ChunkRun);
     WalkRec* walk = reinterpret_cast<WalkRec*>(p);
+    p += (size_t)nimg * nch * sizeof(WalkRec);
+    BatchRec* batches = reinterpret_cast<BatchRec*>(p);
     if (!im1) im1 = im0;
     // the shared-memory limits are set to the bound on every call, never lowered,
     // so concurrent callers cannot race on them
@@ -645,20 +703,20 @@ cudaError_t launch_image_stats(const float* im0, const float* im1, int nimg, siz
                           (const void*)k_stats_sub<1>})
         if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kSegSmemMax);
     if (e != cudaSuccess) return e;
-    const dim3 tgrid((nch + 31) / 32, nimg), cgrid(nch, nimg);
-    k_stats_sums<<<cgrid, 256, 0, s>>>(im0, im1, sz, nch, sx, sx2);
-    k_stats_starts<0><<<nimg, 1024, 0, s>>>(sz, nch, sx, sx2, run);
-    k_stats_traj<0><<<tgrid, 32, 0, s>>>(im0, im1, sz, nch, means, run, walk);
-    k_stats_restarts<0><<<nimg, 1024, 0, s>>>(sz, nch, sx, sx2, run);
-    k_stats_traj<0><<<tgrid, 32, 0, s>>>(im0, im1, sz, nch, means, run, walk);
+    const dim3 tgrid((nch + 31) / 32, nimg), cgrid(nch, nimg), sgrid((nch + 1023) / 1024, nimg);
+    k_stats_sums<<<dim3((nch + 7) / 8, nimg), 256, 0, s>>>(im0, im1, sz, nch, sx, sx2);
+    k_stats_starts<0, false><<<sgrid, 1024, 0, s>>>(sz, nch, sx, sx2, inc, run);
+    k_stats_traj<0><<<tgrid, 32, 0, s>>>(im0, im1, sz, nch, means, inc, run, walk, batches);
+    k_stats_starts<0, true><<<sgrid, 1024, 0, s>>>(sz, nch, sx, sx2, inc, run);
+    k_stats_traj<0><<<tgrid, 32, 0, s>>>(im0, im1, sz, nch, means, inc, run, walk, batches);
     k_stats_sub<0><<<cgrid, 32, seg_smem, s>>>(im0, im1, sz, nch, means, run, sub);
-    k_stats_stitch<0><<<nimg, 32, seg_smem, s>>>(im0, im1, sz, nch, run, walk, sub, means, out);
-    k_stats_starts<1><<<nimg, 1024, 0, s>>>(sz, nch, sx, sx2, run);
-    k_stats_traj<1><<<tgrid, 32, 0, s>>>(im0, im1, sz, nch, means, run, walk);
-    k_stats_restarts<1><<<nimg, 1024, 0, s>>>(sz, nch, sx, sx2, run);
-    k_stats_traj<1><<<tgrid, 32, 0, s>>>(im0, im1, sz, nch, means, run, walk);
+    k_stats_stitch<0><<<nimg, 32, seg_smem, s>>>(im0, im1, sz, nch, run, walk, batches, sub, means, out);
+    k_stats_starts<1, false><<<sgrid, 1024, 0, s>>>(sz, nch, sx, sx2, inc, run);
+    k_stats_traj<1><<<tgrid, 32, 0, s>>>(im0, im1, sz, nch, means, inc, run, walk, batches);
+    k_stats_starts<1, true><<<sgrid, 1024, 0, s>>>(sz, nch, sx, sx2, inc, run);
+    k_stats_traj<1><<<tgrid, 32, 0, s>>>(im0, im1, sz, nch, means, inc, run, walk, batches);
     k_stats_sub<1><<<cgrid, 32, seg_smem, s>>>(im0, im1, sz, nch, means, run, sub);
-    k_stats_stitch<1><<<nimg, 32, seg_smem, s>>>(im0, im1, sz, nch, run, walk, sub, means, out);
+    k_stats_stitch<1><<<nimg, 32, seg_smem, s>>>(im0, im1, sz, nch, run, walk, batches, sub, means, out);
     count_launches(13);
     return cudaGetLastError();
 }
