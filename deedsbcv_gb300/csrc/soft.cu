@@ -1356,6 +1356,8 @@ __device__ __forceinline__ float add_children(const SoftTree& t, int c, const No
     return v;
 }
 
+// The bodies below are for label widths above 9; k_sweep has those up to 9.
+
 // Upward: B_c = C_c + sum_children (M_k - min M_k), stored minus its minimum (the
 // marginals and the parent's (message - min) are invariant to a constant shift of
 // B_c, and the centred values keep the exponents of the label-space transforms
@@ -1669,6 +1671,336 @@ __global__ void k_soft_sweep(SoftTree t, const int* __restrict__ ordered, SweepA
         if (threadIdx.x == 0) {
             if (kTopDown) st_release(st.done + c, 1);
             else if (c != t.root) red_release_add(st.done + t.parents[c], 1);
+        }
+    }
+}
+
+// ---- label widths 3 to 9: one thread per label, the label width known to the compiler
+//
+// A sweep is a chain of dependent nodes (the tree's depth, hundreds at grid 4), so what
+// counts is the time from a finished parent (children) to the next one.  Against the
+// bodies above: the width is a constant (no division, the line's values in registers,
+// one pass for maximum and sum), a block reduction costs one barrier, and everything
+// that does not depend on this sweep is done before the wait; in the two adjoint sweeps
+// that is the whole forward transform and all its weights exp(in - d^2/tau - out), so
+// that behind the wait each axis is LEN products from shared memory.  What no other node
+// reads (displacements, offset gradients) comes after the release.
+// Measured, 343 labels at grid 4: 96x80x112 (13440 nodes) up/down/adjoint down/adjoint up
+// 1.3 to 1.7 ms each before, 0.69/0.69/0.54/0.52 ms now; four pairs of 160x160x192 (76800
+// nodes) in flight together, about 22 ms each before, 9.9/9.7/9.8/6.9 ms now.  The
+// arithmetic and its order are those of the bodies above.  Wider label sets keep those:
+// past 1024 labels there is more than one label per thread.
+template <int LEN>
+struct SweepShared {
+    static constexpr int L2 = LEN * LEN, L3 = LEN * LEN * LEN, W = (L3 + 31) / 32;
+    float x[L3], y[L3], z[L3], w[L3];
+    float red[5][W];
+};
+
+// d(i) = sgn (own - i) + off (forward), sgn (i - own) + off (adjoint)
+__device__ __forceinline__ float fwd_dist(int own, int i, float sgn, float off) { return sgn * (float)(own - i) + off; }
+__device__ __forceinline__ float adj_dist(int own, int i, float sgn, float off) { return sgn * (float)(i - own) + off; }
+
+template <int LEN>
+__device__ __forceinline__ float lse_values(float (&v)[LEN], int own, float itau, float sgn, float off) {
+    float mx = -INFINITY, acc = 0.0f;
+#pragma unroll
+    for (int a = 0; a < LEN; a++) {
+        const float d = fwd_dist(own, a, sgn, off);
+        v[a] -= d * d * itau;
+        mx = fmaxf(mx, v[a]);
+    }
+#pragma unroll
+    for (int a = 0; a < LEN; a++) acc += __expf(v[a] - mx);
+    return mx + __logf(acc);
+}
+
+template <int LEN, int S>
+__device__ __forceinline__ float lse_line(const float* line, int own, float itau, float sgn, float off) {
+    float v[LEN];
+#pragma unroll
+    for (int a = 0; a < LEN; a++) v[a] = line[a * S];
+    return lse_values<LEN>(v, own, itau, sgn, off);
+}
+
+// w[b] = exp(x - d^2/tau - out(b)) along the line
+template <int LEN, int S>
+__device__ __forceinline__ void adj_weights(float (&w)[LEN], float x, const float* out, int own, float itau, float sgn,
+                                            float off) {
+#pragma unroll
+    for (int b = 0; b < LEN; b++) {
+        const float d = adj_dist(own, b, sgn, off);
+        w[b] = __expf(x - d * d * itau - out[b * S]);
+    }
+}
+
+template <int LEN, int S>
+__device__ __forceinline__ float adj_line(const float (&w)[LEN], const float* outbar, int own, float sgn, float off,
+                                          bool want, float& dof) {
+    float wb[LEN], acc = 0.0f;
+#pragma unroll
+    for (int b = 0; b < LEN; b++) wb[b] = outbar[b * S] * w[b];
+#pragma unroll
+    for (int b = 0; b < LEN; b++) acc += wb[b];
+    if (want) {
+#pragma unroll
+        for (int b = 0; b < LEN; b++) dof += wb[b] * adj_dist(own, b, sgn, off);
+    }
+    return acc;
+}
+
+__device__ __forceinline__ float warp_max(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+__device__ __forceinline__ float warp_add(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+// Block reductions with one barrier; red is not written again before two barriers.
+template <int W>
+__device__ __forceinline__ float all_max(float v, float* red) {
+    v = warp_max(v);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    float r = red[0];
+#pragma unroll
+    for (int w = 1; w < W; w++) r = fmaxf(r, red[w]);
+    return r;
+}
+template <int W>
+__device__ __forceinline__ float all_sum(float v, float* red) {
+    v = warp_add(v);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    float r = red[0];
+#pragma unroll
+    for (int w = 1; w < W; w++) r += red[w];
+    return r;
+}
+
+// (max, sum exp(x - max)) of the block; returns the LSE
+template <int W>
+__device__ __forceinline__ float all_lse(float mx, float se, float* rmx, float* rse) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float om = __shfl_xor_sync(0xffffffffu, mx, o), os = __shfl_xor_sync(0xffffffffu, se, o);
+        const float nm = fmaxf(mx, om);
+        se = (mx == -INFINITY ? 0.0f : se * __expf(mx - nm)) + (om == -INFINITY ? 0.0f : os * __expf(om - nm));
+        mx = nm;
+    }
+    if ((threadIdx.x & 31) == 0) {
+        rmx[threadIdx.x >> 5] = mx;
+        rse[threadIdx.x >> 5] = se;
+    }
+    __syncthreads();
+    float m = -INFINITY, t = 0.0f;
+#pragma unroll
+    for (int w = 0; w < W; w++) m = fmaxf(m, rmx[w]);
+#pragma unroll
+    for (int w = 0; w < W; w++)
+        if (rmx[w] != -INFINITY) t += rse[w] * __expf(rmx[w] - m);
+    return m + __logf(t);
+}
+
+template <int KIND, int LEN>
+__global__ void __launch_bounds__(SweepShared<LEN>::W * 32)
+    k_sweep(SoftTree t, const int* __restrict__ ordered, SweepArgs a, SweepState st) {
+    using SH = SweepShared<LEN>;
+    constexpr int L2 = SH::L2, L3 = SH::L3, W = SH::W;
+    constexpr bool kTopDown = KIND == kSweepDown || KIND == kSweepUpAdj;
+    constexpr bool kAdj = KIND == kSweepDownAdj || KIND == kSweepUpAdj;
+    constexpr float sgn = KIND == kSweepUp || KIND == kSweepUpAdj ? 1.0f : -1.0f;
+    __shared__ SH sh;
+    __shared__ int s_tk;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const bool in = tid < L3;
+    const int l = in ? tid : L3 - 1;  // threads past the last label repeat it and write nothing
+    const int ly = l % LEN, lx = (l / LEN) % LEN, lz = l / L2;
+    const int by = l - ly, bx = l - lx * LEN, bz = l - lz * L2;
+    const float itau = t.itau;
+    for (;;) {
+        if (tid == 0) s_tk = atomicAdd(st.ticket, 1);
+        __syncthreads();
+        const int tk = s_tk;
+        if (tk >= t.sz) break;
+        const int c = ordered[kTopDown ? tk : t.sz - 1 - tk];
+        const bool root = c == t.root;
+        const int64_t row = (int64_t)c * L3 + l;
+
+        // ---- before the wait: what earlier sweeps left
+        const int p = root ? c : t.parents[c];
+        const float e = root ? 0.0f : t.edgemst[c];
+        const float oy = edge_off(t, c, 0), ox = edge_off(t, c, 1), oz = edge_off(t, c, 2);
+        NodePre pre;
+        pre.nch = 0;
+        float v0 = 0.0f, v1 = 0.0f;      // own values
+        float wy[LEN], wx[LEN], wz[LEN];  // adjoint weights
+        float gu = 0.0f, gv = 0.0f, gw = 0.0f;
+        if (KIND == kSweepUp) {
+            v0 = a.cost[row];
+            load_children(t, c, pre);
+        } else if (KIND == kSweepDown) {
+            if (!root) v0 = a.M[row];
+            v1 = a.B[row];
+        } else if (KIND == kSweepDownAdj) {
+            v0 = a.logp[row];
+            load_children(t, c, pre);
+            gu = a.gdisp[c];
+            gv = a.gdisp[t.sz + c];
+            gw = a.gdisp[2 * t.sz + c];
+        } else if (!root) {
+            v0 = a.R[row];
+            v1 = a.Bbar[row];
+        }
+        if (kAdj && !root) {
+            const float r = KIND == kSweepDownAdj ? a.logp[(int64_t)p * L3 + l] + a.M[row] * itau
+                                                  : __fmul_rn(-e * a.B[row], itau);
+            if (in) sh.x[tid] = r;
+            __syncthreads();
+            const float t1 = lse_line<LEN, 1>(sh.x + by, ly, itau, sgn, oy);
+            if (in) sh.y[tid] = t1;
+            __syncthreads();
+            const float t2 = lse_line<LEN, LEN>(sh.y + bx, lx, itau, sgn, ox);
+            if (in) sh.z[tid] = t2;
+            __syncthreads();
+            const float t3 = lse_line<LEN, L2>(sh.z + bz, lz, itau, sgn, oz);
+            if (in) sh.w[tid] = t3;
+            __syncthreads();
+            adj_weights<LEN, L2>(wz, t2, sh.w + bz, lz, itau, sgn, oz);
+            adj_weights<LEN, LEN>(wx, t1, sh.z + bx, lx, itau, sgn, ox);
+            adj_weights<LEN, 1>(wy, r, sh.y + by, ly, itau, sgn, oy);
+        }
+        if (tid == 0 && ld_acquire(st.err) == 0) {
+            // top-down: the parent is released (done = 1); bottom-up: every child has arrived
+            const int* flag = kTopDown ? (root ? nullptr : st.done + p) : st.done + c;
+            const int need = kTopDown ? 1 : t.child_ptr[c + 1] - t.child_ptr[c];
+            if (flag && need > 0) bounded_wait_geq(flag, need, st.err);
+        }
+        __syncthreads();
+
+        // ---- between the wait and the release
+        float dof[3] = {0.0f, 0.0f, 0.0f};  // y, x, z
+        float pl = 0.0f;                    // this label's probability (down)
+        if (KIND == kSweepUp) {
+            const float v = add_children(t, c, pre, l, v0, a.M, a.Mmin);
+            if (in) sh.x[tid] = v;
+            const float bmin = -all_max<W>(-v, sh.red[0]);
+            if (in) a.B[row] = v - bmin;
+            if (!root) {
+                float f[LEN];
+#pragma unroll
+                for (int i = 0; i < LEN; i++) f[i] = __fmul_rn(-e * (sh.x[by + i] - bmin), itau);
+                const float t1 = lse_values<LEN>(f, ly, itau, sgn, oy);
+                if (in) sh.y[tid] = t1;
+                __syncthreads();
+                const float t2 = lse_line<LEN, LEN>(sh.y + bx, lx, itau, sgn, ox);
+                if (in) sh.z[tid] = t2;
+                __syncthreads();
+                const float msg = -t.tau * lse_line<LEN, L2>(sh.z + bz, lz, itau, sgn, oz);
+                if (in) a.M[row] = msg;
+                const float mn = -warp_max(-msg);
+                if (lane == 0) sh.red[1][warp] = mn;
+            }
+        } else if (KIND == kSweepDown) {
+            float r;
+            if (root) {
+                r = -v1 * itau;
+            } else {
+                if (in) sh.x[tid] = __ldcg(a.logp + (int64_t)p * L3 + l) + v0 * itau;
+                __syncthreads();
+                const float t1 = lse_line<LEN, 1>(sh.x + by, ly, itau, sgn, oy);
+                if (in) sh.y[tid] = t1;
+                __syncthreads();
+                const float t2 = lse_line<LEN, LEN>(sh.y + bx, lx, itau, sgn, ox);
+                if (in) sh.z[tid] = t2;
+                __syncthreads();
+                r = lse_line<LEN, L2>(sh.z + bz, lz, itau, sgn, oz) - e * v1 * itau;
+            }
+            const float lp = r - all_lse<W>(in ? r : -INFINITY, in ? 1.0f : 0.0f, sh.red[0], sh.red[1]);
+            if (in) a.logp[row] = lp;
+            pl = in ? __expf(lp) : 0.0f;
+        } else if (KIND == kSweepDownAdj) {
+            const float du = (float)((lx - t.hw) * t.q), dv = (float)((ly - t.hw) * t.q), dw = (float)((lz - t.hw) * t.q);
+            const float pc = __expf(v0);
+            const float h = add_children(t, c, pre, l, (gu * du + gv * dv + gw * dw) * pc, a.R, nullptr);
+            if (root) {
+                const float tot = all_sum<W>(in ? h : 0.0f, sh.red[0]);
+                const float b = -(h - pc * tot) * itau;
+                const float mean = all_sum<W>(in ? b : 0.0f, sh.red[1]) / (float)L3;
+                if (in) a.Bbar[row] = b - mean;
+            } else {
+                if (in) {
+                    sh.x[tid] = h;
+                    a.Bbar[row] = -e * itau * h;
+                }
+                __syncthreads();
+                const float gz = adj_line<LEN, L2>(wz, sh.x + bz, lz, sgn, oz, t.offbar, dof[2]);
+                if (in) sh.y[tid] = gz;
+                __syncthreads();
+                const float gx = adj_line<LEN, LEN>(wx, sh.y + bx, lx, sgn, ox, t.offbar, dof[1]);
+                if (in) sh.z[tid] = gx;
+                __syncthreads();
+                const float gy = adj_line<LEN, 1>(wy, sh.z + by, ly, sgn, oy, t.offbar, dof[0]);
+                if (in) a.R[row] = gy;
+            }
+        } else if (!root) {
+            if (in) sh.x[tid] = v0 * itau + __ldcg(a.Bbar + (int64_t)p * L3 + l);
+            __syncthreads();
+            const float gz = adj_line<LEN, L2>(wz, sh.x + bz, lz, sgn, oz, t.offbar, dof[2]);
+            if (in) sh.y[tid] = gz;
+            __syncthreads();
+            const float gx = adj_line<LEN, LEN>(wx, sh.y + bx, lx, sgn, ox, t.offbar, dof[1]);
+            if (in) sh.z[tid] = gx;
+            __syncthreads();
+            const float gy = adj_line<LEN, 1>(wy, sh.z + by, ly, sgn, oy, t.offbar, dof[0]);
+            const float b = v1 + e * gy;
+            const float mean = all_sum<W>(in ? b : 0.0f, sh.red[0]) / (float)L3;
+            if (in) a.Bbar[row] = b - mean;
+        }
+        __syncthreads();
+        if (tid == 0) {
+            if (KIND == kSweepUp && !root) {
+                float mn = sh.red[1][0];
+#pragma unroll
+                for (int w = 1; w < W; w++) mn = fminf(mn, sh.red[1][w]);
+                a.Mmin[c] = mn;
+            }
+            if (kTopDown) st_release(st.done + c, 1);
+            else if (!root) red_release_add(st.done + p, 1);
+        }
+
+        // ---- after the release: sums that no other node reads
+        if (KIND == kSweepDown || (kAdj && t.offbar && !root)) {
+            float s0, s1, s2;  // x, y, z
+            if (KIND == kSweepDown) {
+                s0 = pl * (float)((lx - t.hw) * t.q);
+                s1 = pl * (float)((ly - t.hw) * t.q);
+                s2 = pl * (float)((lz - t.hw) * t.q);
+            } else {
+                // M = -tau out in the upward recursion: its offset gradient scales by -tau
+                const float scale = -2.0f * itau * (KIND == kSweepUpAdj ? -t.tau : 1.0f);
+                s0 = in ? scale * dof[1] : 0.0f;
+                s1 = in ? scale * dof[0] : 0.0f;
+                s2 = in ? scale * dof[2] : 0.0f;
+            }
+            s0 = warp_add(s0);
+            s1 = warp_add(s1);
+            s2 = warp_add(s2);
+            if (lane == 0) {
+                sh.red[2][warp] = s0;
+                sh.red[3][warp] = s1;
+                sh.red[4][warp] = s2;
+            }
+            __syncthreads();
+            if (tid < 3) {
+                float s = 0.0f;
+                for (int w = 0; w < W; w++) s += sh.red[2 + tid][w];
+                if (KIND == kSweepDown) a.disp[(int64_t)tid * t.sz + c] = s;
+                else t.offbar[(int64_t)tid * t.sz + c] += s;
+            }
         }
     }
 }
@@ -1998,20 +2330,29 @@ size_t soft_tree_smem(int len) { return sizeof(float) * (6 * (size_t)len * len *
 template <int KIND>
 static cudaError_t run_sweep(const SoftTree& t, const int* ordered, const SweepArgs& a, const SweepState& st,
                              int* sweep_mem, cudaStream_t s) {
-    const int threads = tree_threads(t.len);
-    const size_t smem = sizeof(float) * ((KIND == kSweepUp || KIND == kSweepDown ? 3 : 6) * (size_t)t.len3 + 96);
-    cudaError_t e = cudaFuncSetAttribute(k_soft_sweep<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
+    int threads = tree_threads(t.len);
+    size_t smem = 0;
+    void (*kern)(SoftTree, const int*, SweepArgs, SweepState) = nullptr;
+    if (t.len == 3) kern = k_sweep<KIND, 3>;
+    else if (t.len == 5) kern = k_sweep<KIND, 5>;
+    else if (t.len == 7) kern = k_sweep<KIND, 7>;
+    else if (t.len == 9) kern = k_sweep<KIND, 9>;
+    else {
+        kern = k_soft_sweep<KIND>;
+        smem = sizeof(float) * ((KIND == kSweepUp || KIND == kSweepDown ? 3 : 6) * (size_t)t.len3 + 96);
+    }
+    cudaError_t e;
+    if (smem && (e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
+        return e;
     int dev = 0, sms = 0, per_sm = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_soft_sweep<KIND>, threads, smem)) != cudaSuccess)
-        return e;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem)) != cudaSuccess) return e;
     per_sm = std::min(per_sm, kSweepCtasPerSm);
     const int grid = std::max(1, std::min(t.sz, sms * std::max(per_sm, 1)));
     // ticket + per-node flags start at zero (the error word is cleared by the caller)
     if ((e = cudaMemsetAsync(sweep_mem, 0, sizeof(int) * ((size_t)t.sz + 1), s)) != cudaSuccess) return e;
-    k_soft_sweep<KIND><<<grid, threads, smem, s>>>(t, ordered, a, st);
+    kern<<<grid, threads, smem, s>>>(t, ordered, a, st);
     count_launches(1);
     return cudaGetLastError();
 }
