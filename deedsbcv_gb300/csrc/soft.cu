@@ -683,7 +683,7 @@ __global__ void __launch_bounds__(256) k_soft_cost_adj_halo(const float* __restr
     }
 }
 
-// Column form of the two halo kernels, for compile-time grid spacing, label width
+// Column form, for compile-time grid spacing, label width
 // and quantisation.  Each node stages a full NA^3 box (NA = g + 2hw*q) of the
 // moving descriptor whose entry (a, b, c) holds the voxel at the clamped
 // coordinates (y*g - hw*q + a, ...): the reference's clamp-to-edge is baked into
@@ -691,8 +691,7 @@ __global__ void __launch_bounds__(256) k_soft_cost_adj_halo(const float* __restr
 // thread owns one sampled column of the node (fixed x and z sample offsets, its g
 // samples along y) and one (lx, lz) label pair, and walks the len y-labels: the
 // displaced y positions i + ly*q of its g samples are NA consecutive box entries,
-// loaded once per channel; in the adjoint each entry's gradient is summed in a
-// register before one shared-memory atomic (instead of one per term).
+// loaded once per channel.
 
 // Block size (whole warps, 128..256) that leaves the fewest idle item slots.
 constexpr int balanced_block(int items) {
@@ -709,9 +708,8 @@ struct ColGeom {
     static constexpr int GS = G_, HW = (LEN_ - 1) / 2, R = HW * Q_, NA = G_ + 2 * R, NA3 = NA * NA * NA;
     static constexpr int S = G_ > 4 ? 2 : 1, NX = (G_ + S - 1) / S, NSAMP = NX * NX * G_;
     static constexpr int ITEMS = NX * NX * LEN_ * LEN_, LEN3 = LEN_ * LEN_ * LEN_;
-    // forward items: (channel half, column, lx, lz); adjoint items per channel group: (channel, column, lx)
-    static constexpr int FWD_ITEMS = 2 * ITEMS, ADJ_ITEMS = 6 * NX * NX * LEN_;
-    static constexpr int FWD_BLOCK = balanced_block(FWD_ITEMS), ADJ_BLOCK = balanced_block(ADJ_ITEMS);
+    // forward items: (channel half, column, lx, lz)
+    static constexpr int FWD_ITEMS = 2 * ITEMS, FWD_BLOCK = balanced_block(FWD_ITEMS);
 };
 
 // Stage channels [c0, c0+CG) of the node's clamped box and, when fs is given, all
@@ -804,116 +802,209 @@ __global__ void __launch_bounds__(ColGeom<G_, LEN_, Q_>::FWD_BLOCK, 4)
         cost[(int64_t)node * CGm::LEN3 + l] = G.alpha1 * (acc[l] - (float)(12 * CGm::NSAMP) * G.eps);
 }
 
-// Adjoint: an item is one (channel, column, lx) of a channel group; it walks lz
-// (different box rows) and, per row, the len y-labels x g samples: the row's
-// gradient sums are accumulated in registers and added to a shared row buffer with
-// one atomic per entry; the column's fixed-side gradients stay in registers across
-// lz and are added once per item.  Channels are processed in two groups of six so
-// that the shared footprint allows four CTAs per SM; items divide the block evenly.
-constexpr int kAdjCG = 6;
+// Two floats in a register pair: one instruction does both lanes' operation, each
+// rounded as the scalar one.
+__device__ __forceinline__ uint64_t f2_pack(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void f2_split(uint64_t v, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
 
-template <int G_, int LEN_, int Q_>
-__global__ void __launch_bounds__(ColGeom<G_, LEN_, Q_>::ADJ_BLOCK, 4)
+// Adjoint of the column form.  A CTA takes one node's half of the channels, a warp one
+// pair of channels (two floats per register pair, as they lie in shared memory), a lane
+// one of the 16 sampled columns; the two half-warps take two label columns (lx, lz) whose
+// box rows (jj + lx, kk + lz) cannot meet: lx or lz four apart.  So a row's gradient is
+// added to shared memory by one lane at a time with plain loads and stores, and the fixed
+// samples with their gradients stay in the lane's registers throughout.
+// Bound by the reciprocal square roots, 16 a clock and SM: at 160x160x192, 343 labels,
+// 20.2 G of them take 4.4 ms (0.78 ms at 96x80x112); 57 % of that rate is reached with the
+// 12 warps an SM has room for.  Shared-memory float adds, a compare-and-swap loop each and
+// 10 of them per 28 terms, took more than the terms: 11.2 ms (2.00 ms) before, 6.9 ms
+// (1.22 ms) now.
+template <int LEN_, int Q_>
+struct AdjGeom {
+    static constexpr int GS = 4, R = (LEN_ - 1) / 2 * Q_, NA = GS + 2 * R, LEN3 = LEN_ * LEN_ * LEN_;
+    static_assert(NA % 2 == 0 && Q_ == 1, "rows are read as 16-byte pairs of entries");
+    // pitches in 16-byte units (two entries): a phase of a 16-byte access is eight lanes,
+    // rows jj = 0..3 of planes kk and kk + 1, which must fall into eight different units
+    static constexpr int RU = NA / 2 % 8 == 4 ? NA / 2 + 1 : NA / 2;
+    static constexpr int ODD = RU % 2;  // odd: the four rows leave a gap of four; even: of one
+    static constexpr int PU = ODD ? (NA * RU + 3) / 8 * 8 + 4 : NA * RU + 1 - NA * RU % 2;
+    static constexpr int CU = NA * PU;  // units of a channel pair
+    static constexpr int WP = (LEN_ + 3) / 4 * 4;
+    // label columns taken two at a time: lx in [0, PX) with lx + 4; the rest by lz
+    static constexpr int PX = LEN_ < 8 ? LEN_ - 4 : 4, NR = LEN_ - 2 * PX;
+    static constexpr int STEPS = PX * LEN_ + NR * (PX + NR);
+    static constexpr size_t SMEM = 16 * (size_t)(6 * CU) + 4 * (size_t)(LEN_ * LEN_ * WP);
+};
+
+template <int LEN_, int Q_>
+__global__ void __launch_bounds__(96)
     k_soft_cost_adj_col(const float* __restrict__ sF, const float* __restrict__ sM, const float* __restrict__ cbar,
                         const float* __restrict__ cost, float* __restrict__ sFbar, float* __restrict__ sMbar,
                         double* __restrict__ dot, SoftGeom G) {
-    using CGm = ColGeom<G_, LEN_, Q_>;
-    extern __shared__ float sh[];
-    __shared__ double red[32];
-    const int node = blockIdx.x;
+    using A = AdjGeom<LEN_, Q_>;
+    extern __shared__ __align__(16) float sh[];
+    __shared__ double red[3];
+    __shared__ int64_t ox[A::NA], oz[A::NA];  // offsets of the box's clamped x and z
+    const int node = blockIdx.x >> 1, half = blockIdx.x & 1;
     const int y = node % G.m1, x = (node / G.m1) % G.n1, z = node / (G.m1 * G.n1);
     const int64_t mn = (int64_t)G.m * G.n, sz = mn * G.o;
-    float* hv = sh;                           // [CG][NA3]
-    float* hg = sh + kAdjCG * CGm::NA3;       // [CG][NA3]
-    float* fs = hg + kAdjCG * CGm::NA3;       // [12][NSAMP]
-    float* gfs = fs + 12 * CGm::NSAMP;        // [12][NSAMP]
-    float* cb = gfs + 12 * CGm::NSAMP;        // [LEN3]
-    const float* cbn = cbar + (int64_t)node * CGm::LEN3;
-    const float* cn = cost + (int64_t)node * CGm::LEN3;
-    // alpha: centred dot product (the exact cbar sums to zero over labels)
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int c0 = 6 * half + 2 * warp;  // this warp's channels c0, c0 + 1
+    float* hv = sh + 4 * A::CU * warp;   // [NA][PU], [NA][RU] of two entries, [2] channels
+    float* hg = hv + 4 * A::CU * 3;
+    float* cb = sh + 4 * A::CU * 6;      // [LEN^2][WP]
+    const int yb = y * 4 - A::R, xb = x * 4 - A::R, zb = z * 4 - A::R;
+    // a warp moves 32/NA box rows at a time: lane -> (row within the group, y offset)
+    constexpr int RPW = 32 / A::NA;
+    const int sub = lane / A::NA, la = lane - sub * A::NA;
+    const int64_t ya = clampi(yb + la, 0, G.m - 1) + (int64_t)c0 * sz;
+    if (threadIdx.x < A::NA) ox[threadIdx.x] = (int64_t)clampi(xb + threadIdx.x, 0, G.n - 1) * G.m;
+    else if (threadIdx.x >= 32 && threadIdx.x < 32 + A::NA)
+        oz[threadIdx.x - 32] = (int64_t)clampi(zb + threadIdx.x - 32, 0, G.o - 1) * mn;
+    __syncthreads();
+    if (sub < RPW)
+#pragma unroll 4
+        for (int b = sub, cc = 0; cc < A::NA;) {
+            const float* g = sM + ya + ox[b] + oz[cc];
+            float* d = hv + 4 * (cc * A::PU + b * A::RU) + 2 * la;
+            cp_async4(d, g);
+            cp_async4(d + 1, g + sz);
+            if ((b += RPW) >= A::NA) {
+                b -= A::NA;
+                cc++;
+            }
+        }
+    for (int e = lane; e < A::CU; e += 32) reinterpret_cast<float4*>(hg)[e] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const float* cbn = cbar + (int64_t)node * A::LEN3;
+    const float* cn = cost + (int64_t)node * A::LEN3;
     double csum = 0.0;
-    for (int l = threadIdx.x; l < CGm::LEN3; l += blockDim.x) {
-        csum += (double)cn[l];
-        cb[l] = cbn[l];
+    for (int l = threadIdx.x; l < A::LEN3; l += 96) {
+        cb[(l / LEN_) * A::WP + l % LEN_] = cbn[l];
+        if (half == 0) csum += (double)cn[l];
     }
-    for (int off = 16; off > 0; off >>= 1) csum += __shfl_xor_sync(0xffffffffu, csum, off);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = csum;
-    for (int e = threadIdx.x; e < 12 * CGm::NSAMP; e += blockDim.x) gfs[e] = 0.0f;
+    // alpha: centred dot product (the exact cbar sums to zero over labels)
+    if (half == 0) {
+        for (int off = 16; off > 0; off >>= 1) csum += __shfl_xor_sync(0xffffffffu, csum, off);
+        if (lane == 0) red[warp] = csum;
+    }
+    // the lane's column: its fixed samples and their gradients
+    const int col = lane & 15, hw = lane >> 4, jj = col & 3, kk = col >> 2;
+    const int64_t fp = (int64_t)c0 * sz + y * 4 + (int64_t)(x * 4 + jj) * G.m + (int64_t)(z * 4 + kk) * mn;
+    uint64_t f[4], gf[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        f[i] = f2_pack(sF[fp + i], sF[fp + i + sz]);
+        gf[i] = 0;
+    }
+    cp_async_wait_all();
     __syncthreads();
-    double cmean = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) cmean += red[w];
-    cmean /= (double)CGm::LEN3;
-    double part = 0.0;
-    for (int l = threadIdx.x; l < CGm::LEN3; l += blockDim.x) part += (double)cb[l] * ((double)cn[l] - cmean);
-    for (int off = 16; off > 0; off >>= 1) part += __shfl_xor_sync(0xffffffffu, part, off);
-    if ((threadIdx.x & 31) == 0) atomicAdd(dot, part);
-    const float eps2 = G.eps * G.eps;
-    const int yb = y * G.g - CGm::R, xb = x * G.g - CGm::R, zb = z * G.g - CGm::R;
-    for (int c0 = 0; c0 < 12; c0 += kAdjCG) {
-        __syncthreads();
-        stage_box<CGm>(G, y, x, z, sM, c0, kAdjCG, hv, sF, c0 == 0 ? fs : nullptr);
-        for (int e = threadIdx.x; e < kAdjCG * CGm::NA3; e += blockDim.x) hg[e] = 0.0f;
-        __syncthreads();
-        // items (column, channel, lx) with the column fastest: a half-warp holds the 16
-        // columns of one (channel, lx), whose box rows (jj + lx, kk + lz) are distinct,
-        // so the row atomics of a warp never collide on an address
-        for (int item = threadIdx.x; item < CGm::ADJ_ITEMS; item += blockDim.x) {
-            const int col = item % (CGm::NX * CGm::NX);
-            const int cl = (item / (CGm::NX * CGm::NX)) % kAdjCG;
-            const int lx = item / (CGm::NX * CGm::NX * kAdjCG);
-            const int jj = col % CGm::NX, kk = col / CGm::NX;
-            const float* fsc = fs + (c0 + cl) * CGm::NSAMP + G_ * col;
-            float f[G_], gf[G_];
+    if (half == 0) {
+        const double cmean = (red[0] + red[1] + red[2]) / (double)A::LEN3;
+        double part = 0.0;
+        for (int l = threadIdx.x; l < A::LEN3; l += 96)
+            part += (double)cb[(l / LEN_) * A::WP + l % LEN_] * ((double)cn[l] - cmean);
+        for (int off = 16; off > 0; off >>= 1) part += __shfl_xor_sync(0xffffffffu, part, off);
+        if (lane == 0) atomicAdd(dot, part);
+    }
+    const uint64_t eps2 = f2_pack(G.eps * G.eps, G.eps * G.eps), minus = f2_pack(-1.0f, -1.0f);
+#pragma unroll 1
+    for (int s = 0; s < A::STEPS; s++) {
+        int lx, lz;
+        bool valid = true;
+        if (s < A::PX * LEN_) {
+            lx = s / LEN_ + 4 * hw;
+            lz = s % LEN_;
+        } else {
+            const int t = s - A::PX * LEN_, r = t / (A::PX + A::NR), u = t % (A::PX + A::NR);
+            lx = LEN_ < 8 ? A::PX + r : 8 + r;
+            lz = u < A::PX ? u + 4 * hw : (LEN_ < 8 ? u : 8 + u - A::PX);
+            valid = u < A::PX || hw == 0;
+        }
+        if (valid) {
+            const int row = (kk + lz) * A::PU + (jj + lx) * A::RU;
+            const ulonglong2* hvr = reinterpret_cast<const ulonglong2*>(hv) + row;
+            ulonglong2* hgr = reinterpret_cast<ulonglong2*>(hg) + row;
+            const float* w = cb + A::WP * (lx + LEN_ * lz);
+            uint64_t v[A::NA], gm[A::NA];
 #pragma unroll
-            for (int i = 0; i < G_; i++) {
-                f[i] = fsc[i];
-                gf[i] = 0.0f;
-            }
-            for (int lz = 0; lz < LEN_; lz++) {
-                const int plane = CGm::NA * ((jj * CGm::S + lx * Q_) + CGm::NA * (kk * CGm::S + lz * Q_));
-                const float* hvr = hv + cl * CGm::NA3 + plane;
-                float* hgr = hg + cl * CGm::NA3 + plane;
-                const float* cbl = cb + LEN_ * (lx + LEN_ * lz);
-                float v[CGm::NA], gm[CGm::NA];
-#pragma unroll
-                for (int a = 0; a < CGm::NA; a++) {
-                    v[a] = hvr[a];
-                    gm[a] = 0.0f;
-                }
-#pragma unroll
-                for (int ly = 0; ly < LEN_; ly++) {
-                    const float w = cbl[ly], nw = -w;
-#pragma unroll
-                    for (int i = 0; i < G_; i++) {
-                        const float d = f[i] - v[i + ly * Q_];
-                        const float t = d * rsqrtf(d * d + eps2);  // phi'(d)
-                        gf[i] = fmaf(w, t, gf[i]);
-                        gm[i + ly * Q_] = fmaf(nw, t, gm[i + ly * Q_]);
-                    }
-                }
-#pragma unroll
-                for (int a = 0; a < CGm::NA; a++) atomicAdd(hgr + a, gm[a]);
+            for (int a = 0; a < A::NA; a += 2) {
+                const ulonglong2 t = hvr[a / 2];
+                v[a] = t.x;
+                v[a + 1] = t.y;
+                gm[a] = gm[a + 1] = 0;
             }
 #pragma unroll
-            for (int i = 0; i < G_; i++) atomicAdd(gfs + (c0 + cl) * CGm::NSAMP + G_ * col + i, gf[i]);
+            for (int ly = 0; ly < LEN_; ly++) {
+                const uint64_t w2 = f2_pack(w[ly], w[ly]);
+                uint64_t d[4], t[4];
+                float q[8];
+#pragma unroll
+                for (int i = 0; i < 4; i++) d[i] = f2_fma(v[i + ly], minus, f[i]);
+#pragma unroll
+                for (int i = 0; i < 4; i++) f2_split(f2_fma(d[i], d[i], eps2), q[2 * i], q[2 * i + 1]);
+#pragma unroll
+                for (int i = 0; i < 8; i++) q[i] = rsqrtf(q[i]);
+#pragma unroll
+                for (int i = 0; i < 4; i++) t[i] = f2_mul(d[i], f2_pack(q[2 * i], q[2 * i + 1]));  // phi'(d)
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    gf[i] = f2_fma(w2, t[i], gf[i]);
+                    gm[i + ly] = f2_fma(w2, t[i], gm[i + ly]);
+                }
+            }
+#pragma unroll
+            for (int a = 0; a < A::NA; a += 2) {
+                ulonglong2 t = hgr[a / 2];
+                t.x = f2_add(t.x, gm[a]);
+                t.y = f2_add(t.y, gm[a + 1]);
+                hgr[a / 2] = t;
+            }
         }
-        __syncthreads();
-        for (int e = threadIdx.x; e < kAdjCG * CGm::NA3; e += blockDim.x) {
-            const float gv = hg[e];
-            if (gv == 0.0f) continue;
-            const int cl = e / CGm::NA3, r = e % CGm::NA3;
-            const int a = r % CGm::NA, b = (r / CGm::NA) % CGm::NA, cc = r / (CGm::NA * CGm::NA);
-            atomicAdd(sMbar + (int64_t)(c0 + cl) * sz + clampi(yb + a, 0, G.m - 1) +
-                          (int64_t)clampi(xb + b, 0, G.n - 1) * G.m + (int64_t)clampi(zb + cc, 0, G.o - 1) * mn,
-                      G.alpha1 * gv);
-        }
+        __syncwarp();  // the next step's rows are other lanes' of this one
     }
-    __syncthreads();
-    for (int e = threadIdx.x; e < 12 * CGm::NSAMP; e += blockDim.x) {
-        const int c = e / CGm::NSAMP, s = e % CGm::NSAMP;
-        const int py = y * G_ + s % G_, px = x * G_ + ((s / G_) % CGm::NX) * CGm::S,
-                  pz = z * G_ + (s / (G_ * CGm::NX)) * CGm::S;
-        sFbar[(int64_t)c * sz + py + (int64_t)px * G.m + (int64_t)pz * mn] = G.alpha1 * gfs[e];
+    // the moving side's gradient is -hg
+    if (sub < RPW)
+#pragma unroll 4
+        for (int b = sub, cc = 0; cc < A::NA;) {
+            const float2 gv = *reinterpret_cast<const float2*>(hg + 4 * (cc * A::PU + b * A::RU) + 2 * la);
+            float* g = sMbar + ya + ox[b] + oz[cc];
+            if (gv.x != 0.0f) atomicAdd(g, -G.alpha1 * gv.x);
+            if (gv.y != 0.0f) atomicAdd(g + sz, -G.alpha1 * gv.y);
+            if ((b += RPW) >= A::NA) {
+                b -= A::NA;
+                cc++;
+            }
+        }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        float g0, g1;
+        f2_split(gf[i], g0, g1);
+        g0 += __shfl_xor_sync(0xffffffffu, g0, 16);
+        g1 += __shfl_xor_sync(0xffffffffu, g1, 16);
+        if (hw == 0) {
+            sFbar[fp + i] = G.alpha1 * g0;
+            sFbar[fp + i + sz] = G.alpha1 * g1;
+        }
     }
 }
 
@@ -1686,8 +1777,8 @@ __global__ void k_soft_sweep(SoftTree t, const int* __restrict__ ordered, SweepA
 // that behind the wait each axis is LEN products from shared memory.  What no other node
 // reads (displacements, offset gradients) comes after the release.
 // Measured, 343 labels at grid 4: 96x80x112 (13440 nodes) up/down/adjoint down/adjoint up
-// 1.3 to 1.7 ms each before, 0.69/0.69/0.54/0.52 ms now; four pairs of 160x160x192 (76800
-// nodes) in flight together, about 22 ms each before, 9.9/9.7/9.8/6.9 ms now.  The
+// 1.3 to 1.7 ms each before, 0.66/0.67/0.56/0.51 ms now; four pairs of 160x160x192 (76800
+// nodes) in flight together, about 22 ms each before, 8.8/8.6/7.3/6.9 ms now (two CTAs to an SM: 9.8 for the third with one).  The
 // arithmetic and its order are those of the bodies above.  Wider label sets keep those:
 // past 1024 labels there is more than one label per thread.
 template <int LEN>
@@ -1806,7 +1897,7 @@ __device__ __forceinline__ float all_lse(float mx, float se, float* rmx, float* 
 }
 
 template <int KIND, int LEN>
-__global__ void __launch_bounds__(SweepShared<LEN>::W * 32)
+__global__ void __launch_bounds__(SweepShared<LEN>::W * 32, LEN <= 7 ? 2 : 1)
     k_sweep(SoftTree t, const int* __restrict__ ordered, SweepArgs a, SweepState st) {
     using SH = SweepShared<LEN>;
     constexpr int L2 = SH::L2, L3 = SH::L3, W = SH::W;
@@ -2147,17 +2238,15 @@ static cudaError_t run_cost_col(const SoftGeom& G, const float* sF, const float*
     return cudaSuccess;
 }
 
-template <int G_, int LEN_, int Q_>
+template <int LEN_, int Q_>
 static cudaError_t run_cost_adj_col(const SoftGeom& G, const float* sF, const float* sM, const float* cbar,
                                     const float* cost, float* sFbar, float* sMbar, double* dot, cudaStream_t st) {
-    using CGm = ColGeom<G_, LEN_, Q_>;
-    const size_t smem = sizeof(float) * (2 * kAdjCG * (size_t)CGm::NA3 + 24 * CGm::NSAMP + CGm::LEN3);
-    if (smem > 200 * 1024) return cudaErrorNotSupported;
-    cudaError_t e = cudaFuncSetAttribute(k_soft_cost_adj_col<G_, LEN_, Q_>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    constexpr size_t smem = AdjGeom<LEN_, Q_>::SMEM;
+    static_assert(smem <= 200 * 1024, "fits an SM");
+    cudaError_t e = cudaFuncSetAttribute(k_soft_cost_adj_col<LEN_, Q_>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)smem);
     if (e != cudaSuccess) return e;
-    k_soft_cost_adj_col<G_, LEN_, Q_><<<G.m1 * G.n1 * G.o1, CGm::ADJ_BLOCK, smem, st>>>(sF, sM, cbar, cost, sFbar,
-                                                                                         sMbar, dot, G);
+    k_soft_cost_adj_col<LEN_, Q_><<<2 * G.m1 * G.n1 * G.o1, 96, smem, st>>>(sF, sM, cbar, cost, sFbar, sMbar, dot, G);
     return cudaSuccess;
 }
 
@@ -2292,9 +2381,9 @@ cudaError_t launch_soft_cost_adj(const float* sF, const float* sM, const float* 
     {
         cudaError_t e = cudaErrorNotSupported;
         switch (col_shape(G)) {
-            case 5: e = run_cost_adj_col<4, 5, 1>(G, sF, sM, cbar, cost, sFbar, sMbar, dot, st); break;
-            case 7: e = run_cost_adj_col<4, 7, 1>(G, sF, sM, cbar, cost, sFbar, sMbar, dot, st); break;
-            case 9: e = run_cost_adj_col<4, 9, 1>(G, sF, sM, cbar, cost, sFbar, sMbar, dot, st); break;
+            case 5: e = run_cost_adj_col<5, 1>(G, sF, sM, cbar, cost, sFbar, sMbar, dot, st); break;
+            case 7: e = run_cost_adj_col<7, 1>(G, sF, sM, cbar, cost, sFbar, sMbar, dot, st); break;
+            case 9: e = run_cost_adj_col<9, 1>(G, sF, sM, cbar, cost, sFbar, sMbar, dot, st); break;
             default: break;
         }
         if (e == cudaSuccess) {
