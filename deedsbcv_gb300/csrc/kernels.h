@@ -128,7 +128,7 @@ size_t soft_tree_smem(int len);
 cudaError_t launch_soft_tree_forward(const SoftTreeDev& d, int* sweep_mem, const float* cost, float* B, float* M,
                                      float* Mmin, float* logp, float* disp, cudaStream_t st);
 cudaError_t launch_soft_tree_backward(const SoftTreeDev& d, int* sweep_mem, const float* B, const float* M,
-                                      const float* logp, const float* gdisp, float* R, float* Bbar, cudaStream_t st);
+                                      const float* logp, const float* gdisp, float* R, float* Bbar, float* Bpart, cudaStream_t st);
 // linearBCV (linear.cu)
 cudaError_t launch_lin_warp(const float* d_in, const float* X, int m, int n, int o, float* d_out, cudaStream_t s);
 cudaError_t launch_lin_smooth(float* d_c0, float* d_c1, int m1, int n1, int o1, int len3, cudaStream_t s);

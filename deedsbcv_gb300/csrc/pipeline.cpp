@@ -1600,12 +1600,13 @@ deeds_status soft_issue_backward(deeds_ctx* ctx, const float* d_fixed, const flo
     }
     float* R = dbuf<float>(ctx, "soft_R", L.sz1 * L.len3, &st);
     float* Bbar = dbuf<float>(ctx, "soft_Bbar", L.sz1 * L.len3, &st);
+    float* Bpart = dbuf<float>(ctx, "soft_Bpart", L.sz1 * L.len3, &st);
     float* sFbar = dbuf<float>(ctx, "soft_sFbar", 12 * L.sz, &st);
     float* sMbar = dbuf<float>(ctx, "soft_sMbar", 12 * L.sz, &st);
     float* dbar6 = dbuf<float>(ctx, "soft_dbar6", 6 * L.sz, &st);
     double* dot = dbuf<double>(ctx, "soft_dot", 1, &st);
     if (st) return st;
-    CK(launch_soft_tree_backward(L.tree, L.sweep, L.B, L.M, L.logp, d_gdisp, R, Bbar, s));
+    CK(launch_soft_tree_backward(L.tree, L.sweep, L.B, L.M, L.logp, d_gdisp, R, Bbar, Bpart, s));
     if (d_gprior) {
         CK(cudaMemsetAsync(d_gprior, 0, sizeof(float) * 3 * L.sz1, s));
         CK(launch_soft_offbar_to_prior(L.tree.offbar, L.tree.parents, L.tree.root, L.sz1, (float)p->quant, d_gprior,

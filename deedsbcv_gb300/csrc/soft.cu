@@ -1666,20 +1666,45 @@ __device__ __forceinline__ void red_release_add(int* p, int v) {
     asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-constexpr long long kSweepSpinLimitV = 1LL << 21;  // ~0.13 s of 64 ns sleeps
+constexpr int kSweepSpinLimit = 1 << 21;  // polls of an L2 round trip each: about a second
 
-// Bounded wait of one thread until *flag >= need; on expiry sets *err and returns
-// false (the caller then skips every further wait).
-__device__ __forceinline__ bool bounded_wait_geq(const int* flag, int need, int* err) {
-    long long it = 0;
-    while (ld_acquire(flag) < need) {
-        if (++it > kSweepSpinLimitV) {
+// Polls until ready(); gives up after the limit (setting *err) or soon after another
+// thread did, and returns false then (the caller carries on with what it has).
+template <class Ready>
+__device__ __forceinline__ bool bounded_poll(Ready ready, int* err) {
+    for (int it = 1; !ready(); it++) {
+        if (it > kSweepSpinLimit) {
             atomicExch(err, 1);
             return false;
         }
-        __nanosleep(64);
+        if (it % 256 == 0 && ld_acquire(err)) return false;
     }
     return true;
+}
+
+__device__ __forceinline__ bool bounded_wait_geq(const int* flag, int need, int* err) {
+    return bounded_poll([&] { return ld_acquire(flag) >= need; }, err);
+}
+
+// A row that other nodes of the same sweep wait for is its own flag: it starts as
+// kNotYet in every word, each word is stored once, and a reader polls the words that
+// it uses.  No word depends on another, so nothing has to be ordered.  (The store never
+// writes kNotYet itself: a NaN with just these bits becomes the usual one.)
+constexpr uint32_t kNotYet = 0xffffffffu;
+
+__device__ __forceinline__ uint32_t ld_word(const float* p) {
+    uint32_t v;
+    asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_word(float* p, float v) {
+    const uint32_t b = __float_as_uint(v);
+    asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(b == kNotYet ? 0x7fffffffu : b) : "memory");
+}
+__device__ __forceinline__ float wait_word(const float* p, int* err) {
+    uint32_t v;
+    bounded_poll([&] { return (v = ld_word(p)) != kNotYet; }, err);
+    return __uint_as_float(v);
 }
 
 struct SweepArgs {
@@ -1692,6 +1717,7 @@ struct SweepArgs {
     const float* gdisp;
     float* R;
     float* Bbar;
+    float* Bpart;  // k_sweep: the downward adjoint's part of Bbar (Bbar itself is waited for)
 };
 
 template <int KIND>
@@ -1775,12 +1801,14 @@ __global__ void k_soft_sweep(SoftTree t, const int* __restrict__ ordered, SweepA
 // that does not depend on this sweep is done before the wait; in the two adjoint sweeps
 // that is the whole forward transform and all its weights exp(in - d^2/tau - out), so
 // that behind the wait each axis is LEN products from shared memory.  What no other node
-// reads (displacements, offset gradients) comes after the release.
-// Measured, 343 labels at grid 4: 96x80x112 (13440 nodes) up/down/adjoint down/adjoint up
-// 1.3 to 1.7 ms each before, 0.66/0.67/0.56/0.51 ms now; four pairs of 160x160x192 (76800
-// nodes) in flight together, about 22 ms each before, 8.8/8.6/7.3/6.9 ms now (two CTAs to an SM: 9.8 for the third with one).  The
-// arithmetic and its order are those of the bodies above.  Wider label sets keep those:
-// past 1024 labels there is more than one label per thread.
+// reads comes last.  A node's row is its own flag (see kNotYet): a round trip to L2 from the
+// parent's store to this node's value, in place of store, fence, flag, poll, barrier, load.
+// Measured, 343 labels at grid 4, up/down/adjoint down/adjoint up.  96x80x112 (13440
+// nodes): the bodies above 1.3 to 1.7 ms each, this form with flags 0.66/0.67/0.56/0.51 ms,
+// with rows as flags 0.46/0.45/0.36/0.35 ms.  Four pairs of 160x160x192 (76800 nodes) in
+// flight together: about 22 ms each, 8.8/8.6/7.3/6.9 ms (one CTA to an SM: 9.8 for the
+// third), 6.1/6.2/5.3/5.0 ms.  The arithmetic and its order are those of the bodies above.
+// Wider label sets keep those: past 1024 labels there is more than one label per thread.
 template <int LEN>
 struct SweepShared {
     static constexpr int L2 = LEN * LEN, L3 = LEN * LEN * LEN, W = (L3 + 31) / 32;
@@ -1850,6 +1878,39 @@ __device__ __forceinline__ float warp_add(float v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
+// v + sum over children in child order of (X[k][l] - xmin[k]) (xmin may be null), each
+// word waited for; up to six children's words are polled together.
+__device__ __forceinline__ float wait_children(const SoftTree& t, int c, const NodePre& pre, int l, float v,
+                                               const float* X, const float* xmin, int* err) {
+    const int L3 = t.len3;
+    if (pre.nch <= kMaxChildren) {
+        uint32_t xs[kMaxChildren], ms[kMaxChildren];
+        bounded_poll([&] {
+            bool ok = true;
+#pragma unroll
+            for (int i = 0; i < kMaxChildren; i++)
+                if (i < pre.nch) {
+                    xs[i] = ld_word(X + (int64_t)pre.ch[i] * L3 + l);
+                    ms[i] = xmin ? ld_word(xmin + pre.ch[i]) : 0u;
+                }
+#pragma unroll
+            for (int i = 0; i < kMaxChildren; i++)
+                if (i < pre.nch) ok = ok && xs[i] != kNotYet && ms[i] != kNotYet;
+            return ok;
+        }, err);
+#pragma unroll
+        for (int i = 0; i < kMaxChildren; i++)
+            if (i < pre.nch) v += xmin ? __uint_as_float(xs[i]) - __uint_as_float(ms[i]) : __uint_as_float(xs[i]);
+        return v;
+    }
+    for (int ci = t.child_ptr[c]; ci < t.child_ptr[c + 1]; ci++) {
+        const int k = t.children[ci];
+        const float x = wait_word(X + (int64_t)k * L3 + l, err);
+        v += xmin ? x - wait_word(xmin + k, err) : x;
+    }
+    return v;
+}
+
 // Block reductions with one barrier; red is not written again before two barriers.
 template <int W>
 __device__ __forceinline__ float all_max(float v, float* red) {
@@ -1905,17 +1966,17 @@ __global__ void __launch_bounds__(SweepShared<LEN>::W * 32, LEN <= 7 ? 2 : 1)
     constexpr bool kAdj = KIND == kSweepDownAdj || KIND == kSweepUpAdj;
     constexpr float sgn = KIND == kSweepUp || KIND == kSweepUpAdj ? 1.0f : -1.0f;
     __shared__ SH sh;
-    __shared__ int s_tk;
+    __shared__ int s_tk[2];  // in turn: the next ticket may be written while this one is being read
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const bool in = tid < L3;
     const int l = in ? tid : L3 - 1;  // threads past the last label repeat it and write nothing
     const int ly = l % LEN, lx = (l / LEN) % LEN, lz = l / L2;
     const int by = l - ly, bx = l - lx * LEN, bz = l - lz * L2;
     const float itau = t.itau;
-    for (;;) {
-        if (tid == 0) s_tk = atomicAdd(st.ticket, 1);
+    for (int turn = 0;; turn ^= 1) {
+        if (tid == 0) s_tk[turn] = atomicAdd(st.ticket, 1);
         __syncthreads();
-        const int tk = s_tk;
+        const int tk = s_tk[turn];
         if (tk >= t.sz) break;
         const int c = ordered[kTopDown ? tk : t.sz - 1 - tk];
         const bool root = c == t.root;
@@ -1944,7 +2005,7 @@ __global__ void __launch_bounds__(SweepShared<LEN>::W * 32, LEN <= 7 ? 2 : 1)
             gw = a.gdisp[2 * t.sz + c];
         } else if (!root) {
             v0 = a.R[row];
-            v1 = a.Bbar[row];
+            v1 = a.Bpart[row];
         }
         if (kAdj && !root) {
             const float r = KIND == kSweepDownAdj ? a.logp[(int64_t)p * L3 + l] + a.M[row] * itau
@@ -1964,19 +2025,11 @@ __global__ void __launch_bounds__(SweepShared<LEN>::W * 32, LEN <= 7 ? 2 : 1)
             adj_weights<LEN, LEN>(wx, t1, sh.z + bx, lx, itau, sgn, ox);
             adj_weights<LEN, 1>(wy, r, sh.y + by, ly, itau, sgn, oy);
         }
-        if (tid == 0 && ld_acquire(st.err) == 0) {
-            // top-down: the parent is released (done = 1); bottom-up: every child has arrived
-            const int* flag = kTopDown ? (root ? nullptr : st.done + p) : st.done + c;
-            const int need = kTopDown ? 1 : t.child_ptr[c + 1] - t.child_ptr[c];
-            if (flag && need > 0) bounded_wait_geq(flag, need, st.err);
-        }
-        __syncthreads();
-
-        // ---- between the wait and the release
+        // ---- what others wait for
         float dof[3] = {0.0f, 0.0f, 0.0f};  // y, x, z
         float pl = 0.0f;                    // this label's probability (down)
         if (KIND == kSweepUp) {
-            const float v = add_children(t, c, pre, l, v0, a.M, a.Mmin);
+            const float v = wait_children(t, c, pre, l, v0, a.M, a.Mmin, st.err);
             if (in) sh.x[tid] = v;
             const float bmin = -all_max<W>(-v, sh.red[0]);
             if (in) a.B[row] = v - bmin;
@@ -1991,7 +2044,7 @@ __global__ void __launch_bounds__(SweepShared<LEN>::W * 32, LEN <= 7 ? 2 : 1)
                 if (in) sh.z[tid] = t2;
                 __syncthreads();
                 const float msg = -t.tau * lse_line<LEN, L2>(sh.z + bz, lz, itau, sgn, oz);
-                if (in) a.M[row] = msg;
+                if (in) st_word(a.M + row, msg);
                 const float mn = -warp_max(-msg);
                 if (lane == 0) sh.red[1][warp] = mn;
             }
@@ -2000,7 +2053,8 @@ __global__ void __launch_bounds__(SweepShared<LEN>::W * 32, LEN <= 7 ? 2 : 1)
             if (root) {
                 r = -v1 * itau;
             } else {
-                if (in) sh.x[tid] = __ldcg(a.logp + (int64_t)p * L3 + l) + v0 * itau;
+                const float x = wait_word(a.logp + (int64_t)p * L3 + l, st.err) + v0 * itau;
+                if (in) sh.x[tid] = x;
                 __syncthreads();
                 const float t1 = lse_line<LEN, 1>(sh.x + by, ly, itau, sgn, oy);
                 if (in) sh.y[tid] = t1;
@@ -2011,12 +2065,12 @@ __global__ void __launch_bounds__(SweepShared<LEN>::W * 32, LEN <= 7 ? 2 : 1)
                 r = lse_line<LEN, L2>(sh.z + bz, lz, itau, sgn, oz) - e * v1 * itau;
             }
             const float lp = r - all_lse<W>(in ? r : -INFINITY, in ? 1.0f : 0.0f, sh.red[0], sh.red[1]);
-            if (in) a.logp[row] = lp;
+            if (in) st_word(a.logp + row, lp);
             pl = in ? __expf(lp) : 0.0f;
         } else if (KIND == kSweepDownAdj) {
             const float du = (float)((lx - t.hw) * t.q), dv = (float)((ly - t.hw) * t.q), dw = (float)((lz - t.hw) * t.q);
             const float pc = __expf(v0);
-            const float h = add_children(t, c, pre, l, (gu * du + gv * dv + gw * dw) * pc, a.R, nullptr);
+            const float h = wait_children(t, c, pre, l, (gu * du + gv * dv + gw * dw) * pc, a.R, nullptr, st.err);
             if (root) {
                 const float tot = all_sum<W>(in ? h : 0.0f, sh.red[0]);
                 const float b = -(h - pc * tot) * itau;
@@ -2025,7 +2079,7 @@ __global__ void __launch_bounds__(SweepShared<LEN>::W * 32, LEN <= 7 ? 2 : 1)
             } else {
                 if (in) {
                     sh.x[tid] = h;
-                    a.Bbar[row] = -e * itau * h;
+                    a.Bpart[row] = -e * itau * h;
                 }
                 __syncthreads();
                 const float gz = adj_line<LEN, L2>(wz, sh.x + bz, lz, sgn, oz, t.offbar, dof[2]);
@@ -2035,10 +2089,11 @@ __global__ void __launch_bounds__(SweepShared<LEN>::W * 32, LEN <= 7 ? 2 : 1)
                 if (in) sh.z[tid] = gx;
                 __syncthreads();
                 const float gy = adj_line<LEN, 1>(wy, sh.z + by, ly, sgn, oy, t.offbar, dof[0]);
-                if (in) a.R[row] = gy;
+                if (in) st_word(a.R + row, gy);
             }
         } else if (!root) {
-            if (in) sh.x[tid] = v0 * itau + __ldcg(a.Bbar + (int64_t)p * L3 + l);
+            const float x = v0 * itau + wait_word(a.Bbar + (int64_t)p * L3 + l, st.err);
+            if (in) sh.x[tid] = x;
             __syncthreads();
             const float gz = adj_line<LEN, L2>(wz, sh.x + bz, lz, sgn, oz, t.offbar, dof[2]);
             if (in) sh.y[tid] = gz;
@@ -2049,21 +2104,19 @@ __global__ void __launch_bounds__(SweepShared<LEN>::W * 32, LEN <= 7 ? 2 : 1)
             const float gy = adj_line<LEN, 1>(wy, sh.z + by, ly, sgn, oy, t.offbar, dof[0]);
             const float b = v1 + e * gy;
             const float mean = all_sum<W>(in ? b : 0.0f, sh.red[0]) / (float)L3;
-            if (in) a.Bbar[row] = b - mean;
+            if (in) st_word(a.Bbar + row, b - mean);
         }
-        __syncthreads();
-        if (tid == 0) {
-            if (KIND == kSweepUp && !root) {
+        if (KIND == kSweepUp && !root) {
+            __syncthreads();
+            if (tid == 0) {
                 float mn = sh.red[1][0];
 #pragma unroll
                 for (int w = 1; w < W; w++) mn = fminf(mn, sh.red[1][w]);
-                a.Mmin[c] = mn;
+                st_word(a.Mmin + c, mn);
             }
-            if (kTopDown) st_release(st.done + c, 1);
-            else if (!root) red_release_add(st.done + p, 1);
         }
 
-        // ---- after the release: sums that no other node reads
+        // ---- sums that no other node reads
         if (KIND == kSweepDown || (kAdj && t.offbar && !root)) {
             float s0, s1, s2;  // x, y, z
             if (KIND == kSweepDown) {
@@ -2419,8 +2472,8 @@ size_t soft_tree_smem(int len) { return sizeof(float) * (6 * (size_t)len * len *
 template <int KIND>
 static cudaError_t run_sweep(const SoftTree& t, const int* ordered, const SweepArgs& a, const SweepState& st,
                              int* sweep_mem, cudaStream_t s) {
-    int threads = tree_threads(t.len);
-    size_t smem = 0;
+    const int threads = tree_threads(t.len);
+    size_t smem = 0, flags = 0;
     void (*kern)(SoftTree, const int*, SweepArgs, SweepState) = nullptr;
     if (t.len == 3) kern = k_sweep<KIND, 3>;
     else if (t.len == 5) kern = k_sweep<KIND, 5>;
@@ -2429,6 +2482,7 @@ static cudaError_t run_sweep(const SoftTree& t, const int* ordered, const SweepA
     else {
         kern = k_soft_sweep<KIND>;
         smem = sizeof(float) * ((KIND == kSweepUp || KIND == kSweepDown ? 3 : 6) * (size_t)t.len3 + 96);
+        flags = t.sz;
     }
     cudaError_t e;
     if (smem && (e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
@@ -2439,8 +2493,21 @@ static cudaError_t run_sweep(const SoftTree& t, const int* ordered, const SweepA
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem)) != cudaSuccess) return e;
     per_sm = std::min(per_sm, kSweepCtasPerSm);
     const int grid = std::max(1, std::min(t.sz, sms * std::max(per_sm, 1)));
-    // ticket + per-node flags start at zero (the error word is cleared by the caller)
-    if ((e = cudaMemsetAsync(sweep_mem, 0, sizeof(int) * ((size_t)t.sz + 1), s)) != cudaSuccess) return e;
+    // the ticket, and the general form's per-node flags, start at zero (the error word is
+    // cleared by the caller); the rows that a sweep waits for start as kNotYet
+    if ((e = cudaMemsetAsync(sweep_mem, 0, sizeof(int) * (flags + 1), s)) != cudaSuccess) return e;
+    if (!flags) {
+        const size_t rows = sizeof(float) * (size_t)t.sz * t.len3;
+        if (KIND == kSweepUp) {
+            if ((e = cudaMemsetAsync(a.M, 0xff, rows, s)) != cudaSuccess) return e;
+            if ((e = cudaMemsetAsync(a.Mmin, 0xff, sizeof(float) * t.sz, s)) != cudaSuccess) return e;
+        } else if (KIND == kSweepDown) {
+            if ((e = cudaMemsetAsync(a.logp, 0xff, rows, s)) != cudaSuccess) return e;
+        } else if (KIND == kSweepDownAdj) {
+            if ((e = cudaMemsetAsync(a.R, 0xff, rows, s)) != cudaSuccess) return e;
+            if ((e = cudaMemsetAsync(a.Bbar, 0xff, rows, s)) != cudaSuccess) return e;
+        }
+    }
     kern<<<grid, threads, smem, s>>>(t, ordered, a, st);
     count_launches(1);
     return cudaGetLastError();
@@ -2449,7 +2516,7 @@ static cudaError_t run_sweep(const SoftTree& t, const int* ordered, const SweepA
 cudaError_t launch_soft_tree_forward(const SoftTreeDev& d, int* sweep_mem, const float* cost, float* B, float* M,
                                      float* Mmin, float* logp, float* disp, cudaStream_t s) {
     const SoftTree t = make_tree(d);
-    SweepArgs a{cost, B, M, Mmin, logp, disp, nullptr, nullptr, nullptr};
+    SweepArgs a{cost, B, M, Mmin, logp, disp, nullptr, nullptr, nullptr, nullptr};
     const SweepState st{sweep_mem, sweep_mem + 1, sweep_mem + t.sz + 1};
     cudaError_t e = run_sweep<kSweepUp>(t, d.ordered, a, st, sweep_mem, s);
     if (e == cudaSuccess) e = run_sweep<kSweepDown>(t, d.ordered, a, st, sweep_mem, s);
@@ -2457,10 +2524,11 @@ cudaError_t launch_soft_tree_forward(const SoftTreeDev& d, int* sweep_mem, const
 }
 
 cudaError_t launch_soft_tree_backward(const SoftTreeDev& d, int* sweep_mem, const float* B, const float* M,
-                                      const float* logp, const float* gdisp, float* R, float* Bbar, cudaStream_t s) {
+                                      const float* logp, const float* gdisp, float* R, float* Bbar, float* Bpart,
+                                      cudaStream_t s) {
     const SoftTree t = make_tree(d);
     SweepArgs a{nullptr, const_cast<float*>(B), const_cast<float*>(M), nullptr, const_cast<float*>(logp), nullptr,
-                gdisp, R, Bbar};
+                gdisp, R, Bbar, Bpart};
     const SweepState st{sweep_mem, sweep_mem + 1, sweep_mem + t.sz + 1};
     cudaError_t e = run_sweep<kSweepDownAdj>(t, d.ordered, a, st, sweep_mem, s);
     if (e == cudaSuccess) e = run_sweep<kSweepUpAdj>(t, d.ordered, a, st, sweep_mem, s);
