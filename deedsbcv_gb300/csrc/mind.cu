@@ -1,19 +1,20 @@
 // MIND-SSC descriptor on sm_103a (replaces descriptor(), src/MINDSSCbox.h:127-232).
 //
 // Layout in HBM: six distance channels D[l][p] (6 x m*n*o float32, context
-// scratch) and the output codes C[p] (uint64).  Four launches:
-//   1. k_pass_i: per (j,k) line and channel, the shifted squared difference
-//      (imshift + distances, src/MINDSSCbox.h:79-124) streamed into the i-axis
-//      box sum, through shared-memory tiles so loads and stores are coalesced;
-//   2. k_pass_jk (j) / 3. k_pass_jk (k): the j- and k-axis box sums, in place;
-//   4. k_quantise: the 12 SSC pairs -> min/mean normalisation -> 5 thresholds
+// scratch) and the output codes C[p] (uint64).  Three launches:
+//   1. k_pass_ij: per slice and channel, the shifted squared difference (imshift +
+//      distances, src/MINDSSCbox.h:79-124) and its box sums along i and j (volumes of
+//      more than 512 lines a slice: k_pass_i and k_pass_jk, one axis each);
+//   2. k_pass_jk (k): the k-axis box sums, in place;
+//   3. k_quantise: the 12 SSC pairs -> min/mean normalisation -> 5 thresholds
 //      -> thermometer code (src/MINDSSCbox.h:175-224).
 // Box sums keep the reference's sequential float prefix sum along each line and
 // its edge rules (src/MINDSSCbox.h:9-73): one thread owns one line and streams it
 // with a lag of r, keeping the last 2r+2 prefix values in a ring; a parallel
 // scan would change the rounding and with it codes near thresholds.
-// Roofline: HBM-bound; per call ~ 4 B read + 24 B write (pass i), 2 x 48 B
-// (passes j, k), 24 B read + 8 B write (quantise) per voxel = 152 B/voxel.
+// Traffic per voxel: 4 B read + 24 B write (pass ij), 48 B (pass k, bound by it), 24 B
+// read + 8 B write (quantise) = 108 B; at 192x160x256 336 us before passes i and j were
+// one and the quantiser counted with integer units, 229 us now.
 #include <cmath>
 
 #include "common.cuh"
@@ -148,6 +149,136 @@ __global__ void __launch_bounds__(6 * TJ) k_pass_i(const float* __restrict__ im,
     }
 }
 
+// i- and j-axis passes in one: CTA = one k slice x one channel, a thread = one line
+// (n <= kIJLines).  The slice is taken in strips of 32 outputs along i: the shifted
+// squared differences of a strip go to shared memory with coalesced loads (lane =
+// sample), each thread runs its line's box sum along the strip in place (prefix and
+// ring stay in its registers from strip to strip; a strip's samples are those QS
+// ahead of its outputs), then the first warp runs the 32 columns' box sums along j and
+// stores them, coalesced along i.  The other warps wait for that one; the CTAs on the
+// SM (six at 160 lines) fill in.
+// D is written once in place of twice and a read, 378 MB less at 192x160x256, where the
+// two passes took 89 + 63 us and this one takes 92 (radius 2; bound by issue, 36
+// instructions a value, and the barriers).  Strips of 64: 116 us (five CTAs, three waves);
+// 48 registers and eight CTAs: 182 us (the loads no longer hit L1); 40: 133 us (spills).
+// Above kIJLines lines a thread would hold several lines' state: those volumes take the
+// two separate passes.
+constexpr int kIJLines = 512, kStrip = 32, kPitch = kStrip + 1;
+
+template <int QS>
+__global__ void __launch_bounds__(kIJLines, 2)
+    k_pass_ij(const float* __restrict__ im, float* __restrict__ D, int m, int n, int o) {
+    extern __shared__ float X[];  // [n][kPitch]
+    const int k = blockIdx.x, l = blockIdx.y;
+    const int64_t mn = (int64_t)m * n;
+    const int dx = c_dx[l] * QS, dy = c_dy[l] * QS, dz = c_dz[l] * QS;
+    const float* slice = im + k * mn;
+    const int away = (int)(dz * mn) + dx * m + dy;  // a partner's distance in samples
+    const bool slice_ok = k + dz < o;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    const int j = threadIdx.x;
+    // squared difference of sample (t, row); a partner outside compares the voxel with itself
+    auto sample = [&](int t, int row) {
+        const int at = row * m + t;
+        const bool ok = slice_ok && (unsigned)(row + dx) < (unsigned)n && (unsigned)(t + dy) < (unsigned)m;
+        const float a = slice[at], d = slice[ok ? at + away : at] - a;
+        return d * d;
+    };
+    float ring[kRing];
+    float P = 0.0f;
+    if (j < n) {
+#pragma unroll
+        for (int t = 0; t < QS; t++) {  // QS < m
+            const float x = sample(t, j);
+            P = t == 0 ? x : P + x;
+            ring[t] = P;
+        }
+    }
+    for (int i0 = 0; i0 < m; i0 += kStrip) {
+        {
+            const int t = min(i0 + QS + lane, m - 1);  // past the line's end: not used
+            const bool ok_t = slice_ok && (unsigned)(t + dy) < (unsigned)m;
+            float* x = X + lane;
+            int row = warp;
+            for (; row + 7 * warps < n; row += 8 * warps) {
+                float a[8], b[8];
+#pragma unroll
+                for (int r = 0; r < 8; r++) {
+                    const int rr = row + r * warps, at = rr * m + t;
+                    a[r] = slice[at];
+                    b[r] = slice[ok_t && (unsigned)(rr + dx) < (unsigned)n ? at + away : at];
+                }
+#pragma unroll
+                for (int r = 0; r < 8; r++) {
+                    const float d = b[r] - a[r];
+                    x[(row + r * warps) * kPitch] = d * d;
+                }
+            }
+            for (; row < n; row += warps) x[row * kPitch] = sample(t, row);
+        }
+        __syncthreads();
+        if (j < n) {
+            float* x = X + j * kPitch;
+            if (i0 > 0 && i0 + kStrip + QS <= m) {  // no line start, no line end
+#pragma unroll
+                for (int u = 0; u < kStrip; u++) {
+                    P = P + x[u];
+                    ring[(QS + u) & (kRing - 1)] = P;
+                    x[u] = P - ring[(u - QS - 1) & (kRing - 1)];
+                }
+            } else {
+#pragma unroll
+                for (int u = 0; u < kStrip; u++) {
+                    const int i = i0 + u;
+                    if (i + QS < m) P = P + x[u];  // past the line's end the prefix stays
+                    ring[(QS + u) & (kRing - 1)] = P;
+                    x[u] = i <= QS ? P : P - ring[(u - QS - 1) & (kRing - 1)];
+                }
+            }
+        }
+        __syncthreads();
+        if (j < kStrip && i0 + j < m) {
+            float* base = D + l * (mn * o) + k * mn + i0 + j;
+            float rj[kRing], Q = 0.0f;
+            for (int c0 = 0; c0 < n; c0 += kRing) {
+                const float* x = X + c0 * kPitch + j;
+                if (c0 > 0 && c0 + kRing < n) {
+                    float* out = base + (int64_t)(c0 - QS) * m;
+                    float y[kRing];
+#pragma unroll
+                    for (int u = 0; u < kRing; u++) y[u] = x[u * kPitch];
+#pragma unroll
+                    for (int u = 0; u < kRing; u++) {
+                        Q = Q + y[u];
+                        rj[u] = Q;
+                        *out = Q - rj[(u - 2 * QS - 1) & (kRing - 1)];
+                        out += m;
+                    }
+                } else {
+#pragma unroll
+                    for (int u = 0; u < kRing; u++) {
+                        const int t = c0 + u;
+                        if (t < n) {
+                            const float y = x[u * kPitch];
+                            Q = t == 0 ? y : Q + y;
+                            rj[u] = Q;
+                            const int jo = t - QS;
+                            if (jo >= 0)
+                                base[(int64_t)jo * m] = jo <= QS ? Q : Q - rj[(u - 2 * QS - 1) & (kRing - 1)];
+                            if (t == n - 1) {
+#pragma unroll
+                                for (int s2 = 0; s2 < QS; s2++)
+                                    base[(int64_t)(n - QS + s2) * m] = Q - rj[(u - 2 * QS + s2) & (kRing - 1)];
+                            }
+                        }
+                    }
+                }
+            }
+        }
+        __syncthreads();  // the strip's tile is consumed
+    }
+}
+
 // In-place box pass along j (axis=1) or k (axis=2); threads over consecutive i.
 // Samples are loaded CHUNK at a time before any of the chunk's outputs (which
 // lag by r) are stored, so the loads of a chunk are independent; with CHUNK a
@@ -202,6 +333,35 @@ struct QuantThr {
 // kSign[l]; a neighbour outside the volume reads the voxel itself.  With QS a
 // compile-time constant every offset is a constant multiple of the line and
 // slice strides and each pair needs one bounds test.
+__device__ __forceinline__ float exp2_approx(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float rcp_approx(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float fmin3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+// RN(x / 12) for finite x >= 0, up to results far below 1e-6: quotient estimate and
+// Markstein's correction by the exact remainder (all 2^23 significands agree with the
+// IEEE division; the exponent only scales).
+__device__ __forceinline__ float twelfth(float x) {
+    const float r = 1.0f / 12.0f, q = __fmul_rn(x, r);
+    return __fmaf_rn(__fmaf_rn(-12.0f, q, x), r, q);
+}
+// `width` ones from bit `pos` on (width >= 0)
+__device__ __forceinline__ uint32_t bit_mask(int pos, int width) {
+    uint32_t r;
+    asm("bmsk.clamp.b32 %0, %1, %2;" : "=r"(r) : "r"(pos), "r"(width));
+    return r;
+}
+
 template <int QS, bool LOGTHR>
 __global__ void __launch_bounds__(64) k_quantise(const float* __restrict__ D, uint64_t* __restrict__ codes, int m,
                                                  int n, int o, QuantThr th) {
@@ -212,26 +372,47 @@ __global__ void __launch_bounds__(64) k_quantise(const float* __restrict__ D, ui
     const int k = blockIdx.z;
     if (i >= m) return;
     const int64_t mn = (int64_t)m * n, sz = mn * o;
-    const int64_t p = i + (int64_t)j * m + k * mn;
-    const float* c = D + p;
-    const bool lo_ok[3] = {i >= QS, j >= QS, k >= QS};
-    const bool hi_ok[3] = {i + QS < m, j + QS < n, k + QS < o};
-    const int64_t step[3] = {QS, (int64_t)QS * m, (int64_t)QS * mn};
+    // a pair's neighbour is in this slice, at a 32-bit index, or at the same place of the
+    // slice QS below, whose base is the block's
+    const uint32_t at = (uint32_t)j * m + i;
+    const uint32_t near[2][2] = {{i >= QS ? at - QS : at, i + QS < m ? at + QS : at},
+                            {j >= QS ? at - QS * m : at, j + QS < n ? at + QS * m : at}};
+    const float* here = D + k * mn;
+    const float* below = k >= QS ? here - QS * mn : here;
+    static_assert(kSign[4] < 0 && kSign[6] < 0 && kSign[8] < 0 && kSign[10] < 0, "k neighbours are below");
     float v[12];
+    auto load = [&]() {
 #pragma unroll
-    for (int l = 0; l < 12; l++) {
-        const int ax = kAxis[l];
-        const bool ok = kSign[l] < 0 ? lo_ok[ax] : hi_ok[ax];
-        const int64_t off = ok ? (kSign[l] < 0 ? -step[ax] : step[ax]) : 0;
-        v[l] = __ldg(c + (l >> 1) * sz + off);
-    }
-    float mn_v = v[0];
-#pragma unroll
-    for (int l = 1; l < 12; l++) mn_v = v[l] < mn_v ? v[l] : mn_v;
+        for (int l = 0; l < 12; l++) {
+            const int ax = kAxis[l];
+            v[l] = ax == 2 ? __ldg(below + (l >> 1) * sz + at) : __ldg(here + (l >> 1) * sz + near[ax][kSign[l] > 0]);
+        }
+    };
+    load();
+    // Finite values: the minimum in any order, and a sum that is below infinity.
     float noise = 0.0f;
+    {
+        float lowest = fmin3(v[0], v[1], v[2]);
 #pragma unroll
-    for (int l = 0; l < 12; l++) { v[l] = v[l] - mn_v; noise = noise + v[l]; }
-    noise = fmaxf(__fdiv_rn(noise, 12.0f), 1e-6f);
+        for (int l = 3; l < 11; l += 2) lowest = fmin3(lowest, v[l], v[l + 1]);
+        lowest = fminf(lowest, v[11]);
+#pragma unroll
+        for (int l = 0; l < 12; l++) { v[l] = v[l] - lowest; noise = noise + v[l]; }
+    }
+    const bool finite = noise < INFINITY;
+    if (!finite) {  // the reference's scan: a NaN first value stays, later ones are skipped
+        load();
+        float lowest = v[0];
+#pragma unroll
+        for (int l = 1; l < 12; l++) lowest = v[l] < lowest ? v[l] : lowest;
+        noise = 0.0f;
+#pragma unroll
+        for (int l = 0; l < 12; l++) { v[l] = v[l] - lowest; noise = noise + v[l]; }
+        noise = __fdiv_rn(noise, 12.0f);
+    } else {
+        noise = twelfth(noise);
+    }
+    noise = fmaxf(noise, 1e-6f);
     // The level only counts the thresholds above the correctly rounded quotient
     // RN(v / noise).  v * RN(1 / noise) is within 1.5 ulp of it (two roundings of
     // at most half an ulp each, relative 2^-24, on a quotient whose own rounding is
@@ -239,53 +420,92 @@ __global__ void __launch_bounds__(64) k_quantise(const float* __restrict__ D, ui
     // that product both give the same count; near a threshold the IEEE division
     // decides.  noise >= 1e-6 (fmaxf drops a NaN sum); NaN, infinite, zero and
     // tiny quotients fall on the same side of every threshold both ways.
-    const float rcp = __frcp_rn(noise);
-    uint64_t code = 0;
+    uint32_t w0 = 0, w1 = 0;  // the code's 60 bits, thermometer {0,1,3,7,15,31} of pair l at bit 5 l
+    auto put = [&](int l, int lvl) {
+        if (l < 6) w0 |= bit_mask(5 * l, lvl);
+        else if (l > 6) w1 |= bit_mask(5 * l - 32, lvl);
+        else {
+            const uint32_t t = bit_mask(0, lvl);
+            w0 |= t << 30;
+            w1 |= t >> 2;
+        }
+    };
+    bool exact = false;
+    if (LOGTHR) {
+        // thresholds -log((c+1.5)/6), c = 0..4: c counts when c < z = 6 exp(-x) - 1.5, so the
+        // level is ceil(z), or 0 below.  z from the fast reciprocal and exponential is within
+        // 2^-17 of the z of the quotient and of the float thresholds: relative errors of
+        // 2^-22 (exponential), 2^-21.4 (its argument) and 2^-20 (thresholds), with y e^-y <=
+        // 0.37, times 6.  One multiply-add places z + 1 at 2^-16 a unit of the mantissa, with
+        // the ceiling above the low 16 bits; where those are within 4 of a whole number for
+        // any pair, or the sum is not finite, the IEEE divisions decide.  (With a rounding, a
+        // ceiling and a conversion for each pair the kernel was bound by the conversion pipe
+        // and by issue, 435 instructions a voxel, 111 us at 192x160x256; now 280 and 72 us.)
+        constexpr float kBase = 192.0f;  // [128, 256): a unit of the last place is 2^-16
+        const float c2 = __fmul_rn(rcp_approx(noise), -1.44269504f);
+        uint32_t z[12], low = 0xffffffffu;
 #pragma unroll
-    for (int l = 0; l < 12; l++) {
-        const float y = __fmul_rn(v[l], rcp);
-        int lvl = 0;
-        bool exact;
-        if (LOGTHR) {
-            // thresholds -log((c+1.5)/6), c = 0..4: c counts when c < z = 6 exp(-x) - 1.5,
-            // so the level is ceil(z) clamped to [0, 5].  z from y and the fast exponential
-            // is within 2^-17 of the z of the quotient and of the float thresholds; within
-            // 2^-12 of an integer (or NaN) the IEEE division decides.
-            const float z = __fadd_rn(__fmul_rn(6.0f, __expf(-y)), -1.5f);
-            exact = !(fabsf(__fsub_rn(z, rintf(z))) >= 0x1p-12f);
-            lvl = min(max((int)ceilf(z), 0), 5);
-        } else {
-            // y outside every threshold's window: each threshold is above or below the
-            // quotient as it is above or below y; y inside a window: the IEEE division decides
-            int cnt = 0;
+        for (int l = 0; l < 12; l++) {
+            const float e = exp2_approx(__fmul_rn(v[l], c2));
+            z[l] = __float_as_uint(__fmaf_rn(6.0f, e, kBase - 1.5f + 1.0f + 4 * 0x1p-16f));
+            put(l, max((int)(z[l] >> 16) - 0x4340, 0));
+        }
+#pragma unroll
+        for (int l = 0; l < 12; l += 4)  // the low halves, two to a word
+            low = __vimin3_u16x2(low, __byte_perm(z[l], z[l + 1], 0x5410), __byte_perm(z[l + 2], z[l + 3], 0x5410));
+        exact = (low & 0xffffu) < 8u || low < 8u << 16 || !finite;
+    } else {
+        // y outside every threshold's window: each threshold is above or below the
+        // quotient as it is above or below y; y inside a window: the IEEE division decides
+        const float rcp = __frcp_rn(noise);
+#pragma unroll
+        for (int l = 0; l < 12; l++) {
+            const float y = __fmul_rn(v[l], rcp);
+            int lvl = 0, cnt = 0;
 #pragma unroll
             for (int q = 0; q < 5; q++) {
                 lvl += y < th.lo[q];
                 cnt += y <= th.hi[q];
             }
-            exact = cnt != lvl;
+            exact = exact || cnt != lvl;
+            put(l, lvl);
         }
-        if (exact) {
+    }
+    if (exact) {
+        w0 = w1 = 0;
+#pragma unroll
+        for (int l = 0; l < 12; l++) {
             const float x = __fdiv_rn(v[l], noise);
-            lvl = 0;
+            int lvl = 0;
 #pragma unroll
             for (int q = 0; q < 5; q++) lvl += th.t[q] > x;
+            put(l, lvl);
         }
-        code |= (uint64_t)((1u << lvl) - 1u) << (5 * l);  // thermometer {0,1,3,7,15,31}
     }
-    codes[p] = code;
+    codes[k * mn + at] = (uint64_t)w1 << 32 | w0;
 }
 
 }  // namespace
 
+// One line per thread, and a partner's distance (up to QS + 1 slices) in 32 bits.
+static bool mind_by_slice(int m, int n) { return n <= kIJLines && (int64_t)m * n < (1 << 28); }
+
 template <int QS>
 static void mind_passes(const float* d_im, int m, int n, int o, const float thr[5], float* d_scratch,
                         uint64_t* d_codes, cudaStream_t s) {
-    const size_t smem = (size_t)(4 * (TJ + 2 * QS) * (CH + 2 * QS + 1) + 6 * TJ * (CH + 1)) * sizeof(float);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_pass_i<QS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_pass_i<QS><<<dim3((n + TJ - 1) / TJ, o), 6 * TJ, smem, s>>>(d_im, d_scratch, m, n, o);
     // 64 i per block: the usual volume extents are multiples of 64, so no lane idles
-    k_pass_jk<QS><<<dim3((m + 63) / 64, o, 6), 64, 0, s>>>(d_scratch, m, n, o, 1);
+    const bool by_slice = mind_by_slice(m, n);
+    if (by_slice) {
+        constexpr int most = kIJLines * kPitch * (int)sizeof(float);
+        cudaFuncSetAttribute(k_pass_ij<QS>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        k_pass_ij<QS><<<dim3(o, 6), (n + 31) / 32 * 32, n * kPitch * sizeof(float), s>>>(d_im, d_scratch, m, n, o);
+    } else {
+        const size_t smem = (size_t)(4 * (TJ + 2 * QS) * (CH + 2 * QS + 1) + 6 * TJ * (CH + 1)) * sizeof(float);
+        if (smem > 48 * 1024)
+            cudaFuncSetAttribute(k_pass_i<QS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        k_pass_i<QS><<<dim3((n + TJ - 1) / TJ, o), 6 * TJ, smem, s>>>(d_im, d_scratch, m, n, o);
+        k_pass_jk<QS><<<dim3((m + 63) / 64, o, 6), 64, 0, s>>>(d_scratch, m, n, o, 1);
+    }
     k_pass_jk<QS><<<dim3((m + 63) / 64, n, 6), 64, 0, s>>>(d_scratch, m, n, o, 2);
     QuantThr th;
     for (int q = 0; q < 5; q++) {
@@ -317,7 +537,7 @@ cudaError_t launch_mind_ssc(const float* d_im, int m, int n, int o, int qs, cons
         case 7: mind_passes<7>(d_im, m, n, o, thr, d_scratch, d_codes, s); break;
         default: return cudaErrorInvalidValue;
     }
-    count_launches(4);
+    count_launches(mind_by_slice(m, n) ? 3 : 4);
     return cudaGetLastError();
 }
 
