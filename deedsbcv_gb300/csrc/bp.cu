@@ -206,6 +206,42 @@ __device__ __forceinline__ void dt_part_val(const float* in, float* out, float o
     }
 }
 
+// The last pass's outputs stay with the thread that made them: o[k] is output I0 + k of
+// its line, label line + (I0 + k) LEN^2.
+template <int LEN, int I0, int I1>
+__device__ __forceinline__ void dt_part_last(const float* in, float* o, float off, int line) {
+    float v[LEN];
+#pragma unroll
+    for (int s = 0; s < LEN; s++) v[s] = in[line + s * LEN * LEN];
+    float z[2 * LEN];
+#pragma unroll
+    for (int u = I0 + 1; u < I1 + LEN; u++) {
+        const float d = (float)(u - LEN) + off;
+        z[u] = d * d;
+    }
+#pragma unroll
+    for (int i = I0; i < I1; i++) {
+        float c[LEN];
+#pragma unroll
+        for (int s = 0; s < LEN; s++) c[s] = v[s] + z[i - s + LEN];
+        const float m = min_all<LEN>(c);
+        o[i - I0] = c[0] != c[0] ? c[0] : m;
+    }
+}
+
+template <int LEN, int P>
+__device__ __forceinline__ void dt_last(int part, const float* in, float* o, float off, int line) {
+    constexpr int K = bp_parts(LEN), OPP = (LEN + K - 1) / K;
+    if constexpr (P < K) {
+        if (part == P) {
+            constexpr int I0 = P * OPP, I1 = (P + 1) * OPP < LEN ? (P + 1) * OPP : LEN;
+            if constexpr (I0 < I1) dt_part_last<LEN, I0, I1>(in, o, off, line);
+            return;
+        }
+        dt_last<LEN, P + 1>(part, in, o, off, line);
+    }
+}
+
 template <int LEN, int AXIS, int P>
 __device__ __forceinline__ void dt_dispatch_val(int part, const float* in, float* out, float off, int base) {
     constexpr int K = bp_parts(LEN), OPP = (LEN + K - 1) / K;
@@ -322,12 +358,16 @@ __global__ void __launch_bounds__(bp_threads(LEN)) k_bp_up(BpTree t, float* __re
                                                            int* __restrict__ err) {
     constexpr int LEN3 = LEN * LEN * LEN;
     constexpr int T = bp_threads(LEN);
-    constexpr int NL = (LEN3 + T - 1) / T;
+    constexpr int LEN2 = LEN * LEN, LP = bp_line_slots(LEN), OPP = (LEN + bp_parts(LEN) - 1) / bp_parts(LEN);
+    // this thread's labels: outputs of its part of its line in the last pass
+    const int part = threadIdx.x / LP, line = threadIdx.x - part * LP;
+    const int first = part * OPP, nl = line < LEN2 ? min(max(LEN - first, 0), OPP) : 0;
+    const int l0 = line + first * LEN2;  // label k: l0 + k LEN^2, k < nl
     extern __shared__ float smem[];
     float* A = smem;
     float* B = A + LEN3;
     int* s_chain = reinterpret_cast<int*>(B + LEN3);  // this chain's finished nodes
-    __shared__ float red[32];
+    __shared__ float red[32], s_first;
     __shared__ int s_node, s_last, s_ready;
     // A thread with no line in the transform passes (the line slots are padded past
     // LEN^2) probes, during the passes, whether the parent's other children have
@@ -383,13 +423,12 @@ __global__ void __launch_bounds__(bp_threads(LEN)) k_bp_up(BpTree t, float* __re
         for (;;) {
             // the parent's row still holds its data cost (it is only written after its
             // own message): load it now, its latency hides behind the transform
-            float acc[NL];
-            const float* prow = cost + (int64_t)p * LEN3;
+            float acc[OPP], msg[OPP];
+            const float* prow = cost + (int64_t)p * LEN3 + l0;
 #pragma unroll
-            for (int k = 0; k < NL; k++) {
-                const int l = tid + k * T;
-                acc[k] = 0.0f;
-                if (l < LEN3) acc[k] = ld_ahead_cg(prow + l);
+            for (int k = 0; k < OPP; k++) {
+                acc[k] = msg[k] = 0.0f;
+                if (k < nl) acc[k] = ld_ahead_cg(prow + k * LEN2);
             }
             // the parent's children (the siblings this step may accumulate)
             int kid[kKidRegs];
@@ -425,32 +464,32 @@ __global__ void __launch_bounds__(bp_threads(LEN)) k_bp_up(BpTree t, float* __re
             dt_lines_val<LEN, 1>(B, A, ox);
             __syncthreads();
             const bool ready = KS > 0 && c1 - c0 > 1 && s_ready;
-            float sib[KS > 0 ? KS : 1][NL], sibm[KS > 0 ? KS : 1];
+            float sib[KS > 0 ? KS : 1][OPP], sibm[KS > 0 ? KS : 1];
 #pragma unroll
             for (int k = 0; k < KS; k++) {
                 if (ready && c0 + k < c1 && kid[k] != node) {
-                    const float* chrow = cost + (int64_t)kid[k] * LEN3;
+                    const float* chrow = cost + (int64_t)kid[k] * LEN3 + l0;
                     sibm[k] = ld_cg(mins + kid[k]);
 #pragma unroll
-                    for (int q = 0; q < NL; q++) {
-                        const int l = tid + q * T;
-                        sib[k][q] = l < LEN3 ? ld_cg(chrow + l) : 0.0f;
-                    }
+                    for (int q = 0; q < OPP; q++) sib[k][q] = q < nl ? ld_cg(chrow + q * LEN2) : 0.0f;
                 }
             }
-            dt_lines_val<LEN, 2>(A, B, oz);  // message in B (its argmins: k_bp_argmin, from `pre`)
-            __syncthreads();
+            if (nl > 0) dt_last<LEN, 0>(part, A, msg, oz, line);  // the message (argmins: k_bp_argmin, from `pre`)
             float mn = INFINITY;
-            float* crow = cost + (int64_t)node * LEN3;
-            for (int l = tid; l < LEN3; l += T) {
-                const float v = B[l];
-                mn = fminf(mn, v);
-                crow[l] = v;
-            }
-            mn = block_min1(mn, red);  // its barrier orders all stores of this CTA before the arrival
+            float* crow = cost + (int64_t)node * LEN3 + l0;
+#pragma unroll
+            for (int k = 0; k < OPP; k++)
+                if (k < nl) {
+                    mn = fminf(mn, msg[k]);
+                    crow[k * LEN2] = msg[k];
+                }
+            if (tid == 0) s_first = msg[0];
+            // its barrier orders all stores of this CTA before the arrival, and every read of A
+            // before the next row is written there
+            mn = block_min1(mn, red);
             // *std::min_element (src/regularisation.h:222) starts from element 0 and only
             // replaces it on '<': a NaN first element is the result, later NaNs are skipped
-            if (isnan(B[0])) mn = B[0];
+            if (isnan(s_first)) mn = s_first;
             if (tid == 0 && lists) {
                 if (s_nchain == kChainSlots) publish_list();
                 s_chain[s_nchain++] = node;
@@ -471,22 +510,17 @@ __global__ void __launch_bounds__(bp_threads(LEN)) k_bp_up(BpTree t, float* __re
                 }
             }
             // the parent's row = data cost + sum over children in MST ordering
-            // order of (message - min); this CTA's own message is still in B
+            // order of (message - min)
             auto add_child = [&](int ch) {
                 if (ch == node) {
 #pragma unroll
-                    for (int k = 0; k < NL; k++) {
-                        const int l = tid + k * T;
-                        if (l < LEN3) acc[k] = acc[k] + (B[l] - mn);
-                    }
+                    for (int k = 0; k < OPP; k++) acc[k] = acc[k] + (msg[k] - mn);
                 } else {
                     const float mch = ld_cg(mins + ch);
-                    const float* chrow = cost + (int64_t)ch * LEN3;
+                    const float* chrow = cost + (int64_t)ch * LEN3 + l0;
 #pragma unroll
-                    for (int k = 0; k < NL; k++) {
-                        const int l = tid + k * T;
-                        if (l < LEN3) acc[k] = acc[k] + (ld_cg(chrow + l) - mch);
-                    }
+                    for (int k = 0; k < OPP; k++)
+                        if (k < nl) acc[k] = acc[k] + (ld_cg(chrow + k * LEN2) - mch);
                 }
             };
 #pragma unroll
@@ -494,10 +528,7 @@ __global__ void __launch_bounds__(bp_threads(LEN)) k_bp_up(BpTree t, float* __re
                 if (c0 + k < c1) {
                     if (k < KS && ready && kid[k] != node) {  // the row loaded during the last pass
 #pragma unroll
-                        for (int q = 0; q < NL; q++) {
-                            const int l = tid + q * T;
-                            if (l < LEN3) acc[q] = acc[q] + (sib[k < KS ? k : 0][q] - sibm[k < KS ? k : 0]);
-                        }
+                        for (int q = 0; q < OPP; q++) acc[q] = acc[q] + (sib[k < KS ? k : 0][q] - sibm[k < KS ? k : 0]);
                     } else {
                         add_child(kid[k]);
                     }
@@ -505,27 +536,22 @@ __global__ void __launch_bounds__(bp_threads(LEN)) k_bp_up(BpTree t, float* __re
             }
             for (int ci = c0 + kKidRegs; ci < c1; ci++) add_child(t.children[ci]);
             if (p == t.root) {
-                float* rrow = cost + (int64_t)p * LEN3;
+                float* rrow = cost + (int64_t)p * LEN3 + l0;
 #pragma unroll
-                for (int k = 0; k < NL; k++) {
-                    const int l = tid + k * T;
-                    if (l < LEN3) rrow[l] = acc[k];
-                }
+                for (int k = 0; k < OPP; k++)
+                    if (k < nl) rrow[k * LEN2] = acc[k];
                 __syncthreads();
                 if (tid == 0 && lists) publish_list();
                 break;
             }
-            __syncthreads();  // B (this message) has been consumed by every thread
-            float* pprow = pre + (int64_t)p * LEN3;
+            float* pprow = pre + (int64_t)p * LEN3 + l0;
 #pragma unroll
-            for (int k = 0; k < NL; k++) {
-                const int l = tid + k * T;
-                if (l < LEN3) {
+            for (int k = 0; k < OPP; k++)
+                if (k < nl) {
                     const float a = __fmul_rn(acc[k], ep);
-                    A[l] = a;
-                    pprow[l] = a;
+                    A[l0 + k * LEN2] = a;
+                    pprow[k * LEN2] = a;
                 }
-            }
             node = p;
             on_x = opx; on_y = opy; on_z = opz;
             p = gp; c0 = gc0; c1 = gc1;
