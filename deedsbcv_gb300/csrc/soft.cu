@@ -81,10 +81,7 @@ __global__ void k_soft_sqdiff(const float* __restrict__ im, float* __restrict__ 
 // directly (no prefix-sum differences, whose cancellation would cost the soft
 // descriptor its float32 accuracy).  The operator is symmetric, so the same
 // kernel is its own adjoint.  Grid: x over i, y over j (32 x 8 blocks), z over
-// (k, channel): no index divisions by runtime sizes.
-// R > 0: compile-time radius (window loads unrolled and issued together); R = 0:
-// the radius r at run time.
-template <int R>
+// (k, channel): no index divisions by runtime sizes.  For radii above 3; below, k_soft_box3.
 __global__ void k_soft_box(const float* __restrict__ in, float* __restrict__ out, int m, int n, int o, int r, int axis) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -99,20 +96,82 @@ __global__ void k_soft_box(const float* __restrict__ in, float* __restrict__ out
     else { L = o; stride = mn; c = k; }
     const float* x = in + (p - (int64_t)c * stride);
     float acc = 0.0f;
-    if (R > 0) {
-        float v[2 * R + 1];
+    const int a0 = max(0, c - r), a1 = min(L - 1, c + r);
+    for (int a = a0; a <= a1; a++) acc += x[a * stride];
+    out[p] = acc;
+}
+
+// The three windowed sums in one pass, radius R (a compile-time constant, up to 3), of
+// six channels: of `in` (6 x sz), or (IMAGE) of the squared differences of k_soft_sqdiff
+// made from the image `in` on the way.  A block marches along k over 32 x 8 columns: each
+// plane's tile and halo go to shared memory (double-buffered, one barrier a plane, the
+// next plane's loads in flight), a thread sums its window along i, then j, and keeps
+// the last 2R + 1 planes' sums in registers for k.  Sums and their order are those of the
+// three passes.  Bound by issue (about 50 instructions a value at R = 1).
+// 96x80x112, radius 1: differences and three passes 73 us, one launch 29; three passes of
+// given channels 63 us, one launch 16.
+constexpr int kBoxPlanes = 32;  // planes a block outputs: 2R more are read
+
+template <int R, bool IMAGE>
+__global__ void __launch_bounds__(256) k_soft_box3(const float* __restrict__ in, float* __restrict__ out, int m, int n,
+                                                   int o, int qs) {
+    constexpr int TI = 32, TJ = 8, SI = TI + 2 * R, SJ = TJ + 2 * R, NE = (SI * SJ + 255) / 256;
+    __shared__ float tile[2][SJ][SI];
+    const int ch = blockIdx.z % 6, k0 = (int)(blockIdx.z / 6) * kBoxPlanes, k1 = min(o, k0 + kBoxPlanes);
+    const int64_t mn = (int64_t)m * n, sz = mn * o;
+    const float* vol = IMAGE ? in : in + ch * sz;
+    const int ti = threadIdx.x % TI, tj = threadIdx.x / TI;
+    const int i = blockIdx.x * TI + ti, j = blockIdx.y * TJ + tj;
+    const int di = IMAGE ? s_dy[ch] * qs : 0, dj = IMAGE ? s_dx[ch] * qs : 0, dk = IMAGE ? s_dz[ch] * qs : 0;
+    float next[NE];
+    auto fetch = [&](int k) {
 #pragma unroll
-        for (int d = -R; d <= R; d++) {
-            const int a = c + d;
-            v[d + R] = (a >= 0 && a < L) ? __ldg(x + a * stride) : 0.0f;
+        for (int e = 0; e < NE; e++) {
+            const int at = threadIdx.x + e * 256, b = at / SI, a = at - b * SI;
+            const int ii = blockIdx.x * TI - R + a, jj = blockIdx.y * TJ - R + b;
+            float v = 0.0f;
+            if (at < SI * SJ && inside(ii, jj, k, m, n, o)) {
+                const int64_t p = ii + (int64_t)jj * m + k * mn;
+                v = __ldg(vol + p);
+                if (IMAGE) {
+                    const bool both = inside(ii + di, jj + dj, k + dk, m, n, o);
+                    const float d = both ? __ldg(vol + p + di + (int64_t)dj * m + dk * mn) - v : 0.0f;
+                    v = d * d;
+                }
+            }
+            next[e] = v;
+        }
+    };
+    float win[2 * R + 1];
+#pragma unroll
+    for (int d = 0; d <= 2 * R; d++) win[d] = 0.0f;
+    fetch(k0 - R);
+    for (int k = k0 - R, buf = 0; k < k1 + R; k++, buf ^= 1) {
+#pragma unroll
+        for (int e = 0; e < NE; e++) {
+            const int at = threadIdx.x + e * 256;
+            if (at < SI * SJ) tile[buf][0][at] = next[e];
+        }
+        __syncthreads();
+        if (k + 1 < k1 + R) fetch(k + 1);
+        float sj = 0.0f;
+#pragma unroll
+        for (int b = 0; b <= 2 * R; b++) {
+            float si = 0.0f;
+#pragma unroll
+            for (int a = 0; a <= 2 * R; a++) si += tile[buf][tj + b][ti + a];
+            sj += si;
         }
 #pragma unroll
-        for (int d = 0; d <= 2 * R; d++) acc += v[d];
-    } else {
-        const int a0 = max(0, c - r), a1 = min(L - 1, c + r);
-        for (int a = a0; a <= a1; a++) acc += x[a * stride];
+        for (int d = 0; d < 2 * R; d++) win[d] = win[d + 1];
+        win[2 * R] = sj;
+        if (k - R >= k0 && i < m && j < n) {
+            float acc = 0.0f;
+#pragma unroll
+            for (int d = 0; d <= 2 * R; d++) acc += win[d];
+            out[ch * sz + i + (int64_t)j * m + (k - R) * mn] = acc;
+        }
     }
-    out[p] = acc;
 }
 
 struct DescPoint {
@@ -2205,22 +2264,29 @@ __global__ void k_soft_offbar_to_prior(const float* __restrict__ offbar, const i
 // ---------------------------------------------------------------------------
 // Host drivers
 
-// three box passes a -> b -> a -> b; the result is in b
-template <int R>
-static void box3_r(float* a, float* b, int m, int n, int o, int r, cudaStream_t st) {
-    const dim3 blk(32, 8), grid(blocks_for(m, 32), blocks_for(n, 8), 6 * o);
-    k_soft_box<R><<<grid, blk, 0, st>>>(a, b, m, n, o, r, 0);
-    k_soft_box<R><<<grid, blk, 0, st>>>(b, a, m, n, o, r, 1);
-    k_soft_box<R><<<grid, blk, 0, st>>>(a, b, m, n, o, r, 2);
-}
-
-static void box3(float* a, float* b, int m, int n, int o, int r, cudaStream_t st) {
-    switch (r) {
-        case 1: box3_r<1>(a, b, m, n, o, r, st); break;
-        case 2: box3_r<2>(a, b, m, n, o, r, st); break;
-        case 3: box3_r<3>(a, b, m, n, o, r, st); break;
-        default: box3_r<0>(a, b, m, n, o, r, st); break;
+// The windowed sums of six channels into b: of the channels in a, or with an image of its
+// squared differences (a is scratch for radii above 3).  Counts its launches.
+static void box3(const float* image, float* a, float* b, int m, int n, int o, int r, cudaStream_t st) {
+    const dim3 blk3(blocks_for(m, 32), blocks_for(n, 8), 6 * blocks_for(o, kBoxPlanes));
+    switch (image ? -r : r) {
+        case -1: k_soft_box3<1, true><<<blk3, 256, 0, st>>>(image, b, m, n, o, r); count_launches(1); return;
+        case -2: k_soft_box3<2, true><<<blk3, 256, 0, st>>>(image, b, m, n, o, r); count_launches(1); return;
+        case -3: k_soft_box3<3, true><<<blk3, 256, 0, st>>>(image, b, m, n, o, r); count_launches(1); return;
+        case 1: k_soft_box3<1, false><<<blk3, 256, 0, st>>>(a, b, m, n, o, r); count_launches(1); return;
+        case 2: k_soft_box3<2, false><<<blk3, 256, 0, st>>>(a, b, m, n, o, r); count_launches(1); return;
+        case 3: k_soft_box3<3, false><<<blk3, 256, 0, st>>>(a, b, m, n, o, r); count_launches(1); return;
+        default: break;
     }
+    if (image) {
+        const int64_t sz = (int64_t)m * n * o;
+        k_soft_sqdiff<<<blocks_for(sz, 256), 256, 0, st>>>(image, a, m, n, o, r);
+        count_launches(1);
+    }
+    const dim3 blk(32, 8), grid(blocks_for(m, 32), blocks_for(n, 8), 6 * o);
+    k_soft_box<<<grid, blk, 0, st>>>(a, b, m, n, o, r, 0);
+    k_soft_box<<<grid, blk, 0, st>>>(b, a, m, n, o, r, 1);
+    k_soft_box<<<grid, blk, 0, st>>>(a, b, m, n, o, r, 2);
+    count_launches(3);
 }
 
 cudaError_t launch_soft_offsets(const float* prior, const int* parents, int root, int sz, float q, float* off,
@@ -2240,24 +2306,22 @@ cudaError_t launch_soft_offbar_to_prior(const float* offbar, const int* parents,
 cudaError_t launch_soft_descriptor(const float* d_im, float* w6a, float* w6b, float* s12, int m, int n, int o, int qs,
                                    cudaStream_t st) {
     const int64_t sz = (int64_t)m * n * o;
-    k_soft_sqdiff<<<blocks_for(sz, 256), 256, 0, st>>>(d_im, w6a, m, n, o, qs);
-    box3(w6a, w6b, m, n, o, qs, st);
+    box3(d_im, w6a, w6b, m, n, o, qs, st);
     k_soft_desc<<<blocks_for(sz, 256), 256, 0, st>>>(w6b, s12, m, n, o, qs);
-    count_launches(5);
+    count_launches(1);
     return cudaGetLastError();
 }
 
 cudaError_t launch_soft_descriptor_adj(const float* d_im, float* w6a, float* w6b, const float* sbar12, float* dbar6,
                                        float* imbar, int m, int n, int o, int qs, cudaStream_t st) {
     const int64_t sz = (int64_t)m * n * o;
-    k_soft_sqdiff<<<blocks_for(sz, 256), 256, 0, st>>>(d_im, w6a, m, n, o, qs);
-    box3(w6a, w6b, m, n, o, qs, st);
+    box3(d_im, w6a, w6b, m, n, o, qs, st);
     cudaError_t err = cudaMemsetAsync(dbar6, 0, sizeof(float) * 6 * sz, st);
     if (err != cudaSuccess) return err;
     k_soft_desc_adj<<<blocks_for(sz, 256), 256, 0, st>>>(w6b, sbar12, dbar6, m, n, o, qs);
-    box3(dbar6, w6b, m, n, o, qs, st);  // adjoint of the box filter: the same operator
+    box3(nullptr, dbar6, w6b, m, n, o, qs, st);  // adjoint of the box filter: the same operator
     k_soft_sqdiff_adj<<<blocks_for(sz, 256), 256, 0, st>>>(d_im, w6b, imbar, m, n, o, qs);
-    count_launches(9);
+    count_launches(2);
     return cudaGetLastError();
 }
 
