@@ -44,7 +44,7 @@ METRIC = "pairs/s at 192x160x256 (5 levels)"
 # beside the algorithmic bytes of the same launch as `achieved` counts them
 # (k_bp_up: the 122,880 x 729 float cost volume read and its message rows
 # written; k_data_cost_mma: both code volumes read once, the cost volume written).
-TRAFFIC = {"k_bp_up": 1030865536, "k_data_cost_mma": 1614965248}
+TRAFFIC = {"k_bp_up": 1029424768, "k_data_cost_mma": 422125440}
 TRAFFIC_ALGORITHMIC = {"k_bp_up": 2 * 122880 * 729 * 4, "k_data_cost_mma": 2 * 192 * 160 * 256 * 8 + 122880 * 729 * 4}
 TRAFFIC_NOTE = ("finest-level launch (grid 4) at 192x160x256, ncu dram__bytes_read.sum + dram__bytes_write.sum; "
                 "k_bp_up also writes each node's scaled input row, which the downward pass reads to evaluate "

@@ -447,7 +447,7 @@ deeds_status deeds_estimate_affine_dev(deeds_ctx* ctx, const float* d_fixed, con
 deeds_status deeds_affine_robust(const float* pts1, const float* pts2, int len, int rigid, float RT[16]);
 
 /* Self-test of the bounded device-side waits: the tree sweeps' wait on a flag and
- * the cost volume's wait on a TMA mbarrier are each run on a flag / barrier that
+ * the cost volume's wait on an mbarrier are each run on a flag / barrier that
  * nothing releases; *sweep_gave_up / *tma_gave_up are set to 1 when the wait
  * expired and reported it (the error word for the sweep), *seconds to the time
  * both took.  The context stays usable afterwards. */
