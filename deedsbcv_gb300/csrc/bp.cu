@@ -267,13 +267,14 @@ __device__ __forceinline__ void dt_lines_val(const float* in, float* out, float 
 // Block-wide minimum with one barrier: warps reduce by shuffles, then every thread
 // reduces the per-warp values.  `red` must not be rewritten before every thread has
 // read it (the caller's next barrier).
+template <int NW>
 __device__ __forceinline__ float block_min1(float v, float* red) {
     for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
     __syncthreads();
-    const int nw = (int)(blockDim.x >> 5);
     v = red[0];
-    for (int w = 1; w < nw; w++) v = fminf(v, red[w]);
+#pragma unroll
+    for (int w = 1; w < NW; w++) v = fminf(v, red[w]);  // the loads together, not one after another
     return v;
 }
 
@@ -486,7 +487,7 @@ __global__ void __launch_bounds__(bp_threads(LEN)) k_bp_up(BpTree t, float* __re
             if (tid == 0) s_first = msg[0];
             // its barrier orders all stores of this CTA before the arrival, and every read of A
             // before the next row is written there
-            mn = block_min1(mn, red);
+            mn = block_min1<T / 32>(mn, red);
             // *std::min_element (src/regularisation.h:222) starts from element 0 and only
             // replaces it on '<': a NaN first element is the result, later NaNs are skipped
             if (isnan(s_first)) mn = s_first;
