@@ -227,6 +227,8 @@ __device__ __forceinline__ bool int_blend8(float dx, float dy, float dz, float c
     const float fx = dx * 32.0f, fy = dy * 32.0f, fz = dz * 32.0f;
     const int ix = (int)fx, iy = (int)fy, iz = (int)fz;
     if ((float)ix != fx || (float)iy != fy || (float)iz != fz) return false;
+    // a coordinate beyond the integers leaves a fraction outside [0, 1]: not these sums' range
+    if ((unsigned)ix > 32u || (unsigned)iy > 32u || (unsigned)iz > 32u) return false;
     const float c[8] = {c000, c100, c010, c001, c110, c101, c011, __fmul_rn(dx * dy * dz, c111)};
     uint32_t e_lo = 255u, e_hi = 0u;
 #pragma unroll
