@@ -67,12 +67,19 @@ __device__ __forceinline__ float blend8_apply(const Blend8Weights& b, float c000
     return (float)acc;
 }
 
-// Corner offsets of a clamp-to-edge trilinear sample at integer corner (y,x,z).
+// Corner offsets of a clamp-to-edge trilinear sample at integer corner (y,x,z).  The
+// corner comes from a float coordinate of any value (an infinite one is the largest
+// integer), so it is brought to -1..size first: the edge voxels are the same, and adding
+// 1 to it cannot overflow.  (An overflowing sum has no defined value; the offsets made
+// from one left the volume.)
 struct Corners {
     int64_t o000, o100, o010, o001, o110, o101, o011, o111;
 };
 
 __device__ __forceinline__ Corners corners(int y, int x, int z, int m2, int n2, int o2) {
+    y = clampi(y, -1, m2);
+    x = clampi(x, -1, n2);
+    z = clampi(z, -1, o2);
     const int y0 = clampi(y, 0, m2 - 1), y1 = clampi(y + 1, 0, m2 - 1);
     const int x0 = clampi(x, 0, n2 - 1), x1 = clampi(x + 1, 0, n2 - 1);
     const int z0 = clampi(z, 0, o2 - 1), z1 = clampi(z + 1, 0, o2 - 1);
@@ -88,6 +95,10 @@ __device__ __forceinline__ Corners corners(int y, int x, int z, int m2, int n2, 
     c.o111 = y1 + x1 * s1 + z1 * s2;
     return c;
 }
+
+// base + d along an axis of `size` voxels, base one of them: beyond the volume on d's side
+// wherever base + d would be, without overflow.
+__device__ __forceinline__ int displaced(int base, int d, int size) { return base + clampi(d, -size, size); }
 
 __device__ __forceinline__ float sample(const float* __restrict__ v, const Corners& c, const Blend8Weights& b) {
     return blend8_apply(b, __ldg(v + c.o000), __ldg(v + c.o100), __ldg(v + c.o010), __ldg(v + c.o001),
@@ -225,7 +236,7 @@ __device__ __forceinline__ bool ff_blend8(const FFWeights& b, float c000, float 
 __device__ __forceinline__ bool int_blend8(float dx, float dy, float dz, float c000, float c100, float c010, float c001,
                                            float c110, float c101, float c011, float c111, float& out) {
     const float fx = dx * 32.0f, fy = dy * 32.0f, fz = dz * 32.0f;
-    const int ix = (int)fx, iy = (int)fy, iz = (int)fz;
+    const int ix = __float2int_rz(fx), iy = __float2int_rz(fy), iz = __float2int_rz(fz);
     if ((float)ix != fx || (float)iy != fy || (float)iz != fz) return false;
     // a coordinate beyond the integers leaves a fraction outside [0, 1]: not these sums' range
     if ((unsigned)ix > 32u || (unsigned)iy > 32u || (unsigned)iz > 32u) return false;
@@ -281,9 +292,10 @@ __device__ __forceinline__ float sample_ff(const float* __restrict__ v, const Co
 }
 
 // Split a float coordinate into floor (as int) and fraction, as `int x=floor(x1);
-// float dx=x1-x;` does in the reference.
+// float dx=x1-x;` does in the reference.  (The intrinsic, because a cast has no defined
+// result beyond the integers; it gives the nearest one, and 0 for NaN.)
 __device__ __forceinline__ void split_coord(float c, int& i, float& f) {
-    i = (int)floorf(c);
+    i = __float2int_rd(c);
     f = c - (float)i;
 }
 

@@ -25,7 +25,7 @@ __device__ __forceinline__ Axis axis_at(float c, int size) {
     const float fl = floorf(c);
     Axis a;
     a.f = c - fl;
-    const int i = (int)fl;
+    const int i = clampi(__float2int_rd(c), -1, size);  // the same corners; i + 1 cannot overflow (an infinite c)
     a.i0 = clampi(i, 0, size - 1);
     a.i1 = clampi(i + 1, 0, size - 1);
     return a;

@@ -237,7 +237,8 @@ __global__ void k_warp_image(const float* __restrict__ in, Grid3 g, const float*
         split_coord(u, x, dx);
         split_coord(v, y, dy);
         split_coord(w, z, dz);
-        out[p] = sample_ff(in, corners(y + i, x + j, z + k, m, n, o), ff_weights(dx, dy, dz), dx, dy, dz);
+        const Corners c = corners(displaced(i, y, m), displaced(j, x, n), displaced(k, z, o), m, n, o);
+        out[p] = sample_ff(in, c, ff_weights(dx, dy, dz), dx, dy, dz);
     });
 }
 
@@ -253,7 +254,7 @@ __global__ void k_warp_seg(const short* __restrict__ in, Affine12 X, Grid3 g, co
         const float y1 = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(fi, X.x[0]), __fmul_rn(fj, X.x[1])), __fmul_rn(fk, X.x[2])), X.x[3]), v);
         const float x1 = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(fi, X.x[4]), __fmul_rn(fj, X.x[5])), __fmul_rn(fk, X.x[6])), X.x[7]), u);
         const float z1 = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(fi, X.x[8]), __fmul_rn(fj, X.x[9])), __fmul_rn(fk, X.x[10])), X.x[11]), w);
-        const int x = (int)roundf(x1), y = (int)roundf(y1), z = (int)roundf(z1);
+        const int x = __float2int_rz(roundf(x1)), y = __float2int_rz(roundf(y1)), z = __float2int_rz(roundf(z1));
         out[p] = in[clampi(y, 0, m - 1) + (int64_t)clampi(x, 0, n - 1) * m + (int64_t)clampi(z, 0, o - 1) * (int64_t)m * n];
     });
 }
@@ -295,7 +296,7 @@ __global__ void k_consistent_step(const float* __restrict__ us, const float* __r
         split_coord(us[p], x, dx);
         split_coord(vs[p], y, dy);
         split_coord(ws[p], z, dz);
-        const Corners c = corners(y + i, x + j, z + k, m, n, o);
+        const Corners c = corners(displaced(i, y, m), displaced(j, x, n), displaced(k, z, o), m, n, o);
         const FFWeights b = ff_weights(dx, dy, dz);
         nu[p] = half_difference(us[p], sample_ff(us2, c, b, dx, dy, dz));
         nv[p] = half_difference(vs[p], sample_ff(vs2, c, b, dx, dy, dz));
@@ -307,7 +308,7 @@ __global__ void k_consistent_step(const float* __restrict__ us, const float* __r
         split_coord(us2[p], x, dx);
         split_coord(vs2[p], y, dy);
         split_coord(ws2[p], z, dz);
-        const Corners c = corners(y + i, x + j, z + k, m, n, o);
+        const Corners c = corners(displaced(i, y, m), displaced(j, x, n), displaced(k, z, o), m, n, o);
         const FFWeights b = ff_weights(dx, dy, dz);
         nu2[p] = half_difference(us2[p], sample_ff(us, c, b, dx, dy, dz));
         nv2[p] = half_difference(vs2[p], sample_ff(vs, c, b, dx, dy, dz));
