@@ -112,7 +112,7 @@ __device__ __forceinline__ float sample(const float* __restrict__ v, const Corne
 // weight factors 1-d (double), exact products of two of them, one rounded
 // product per weight, eight rounded products with the corner values, seven
 // rounded sums, one float term (dx*dy*dz*c111) and a final rounding to float.
-// With S = sum of |corner values| (weights are at most 1), its double result
+// With S = sum of |corner values| (weights are at most 1: fractions in [0, 1]), its double result
 // differs from the exact value of the expression by at most ~2^-49.8 S (each of
 // the ~16 double roundings adds at most 2^-53 of an intermediate bounded by S).
 // The float-float evaluation below (Dekker/Knuth error-free sum and product
@@ -121,7 +121,7 @@ __device__ __forceinline__ float sample(const float* __restrict__ v, const Corne
 // the two differ by less than eps = 2^-40 S.  If the float-float value lies
 // farther than eps from every midpoint between adjacent floats, both round to
 // the same float, and that float is returned; otherwise (a value near a
-// midpoint, non-finite or very small or large inputs) ff_blend8 reports failure
+// midpoint, other fractions, non-finite or very small or large inputs) ff_blend8 reports failure
 // and the caller evaluates blend8_apply.
 struct FF {
     float hi, lo;
@@ -179,6 +179,7 @@ __device__ __forceinline__ bool ff_round_safe(FF acc, float eps, float& out) {
 struct FFWeights {
     FF w000, w100, w010, w001, w110, w101, w011;
     float dxdydz;
+    float eps;  // the evaluation's error over S: infinite for fractions outside [0, 1]
 };
 
 // The weights of blend8_weights in float-float (the same factors and products).
@@ -197,6 +198,10 @@ __device__ __forceinline__ FFWeights ff_weights(float dx, float dy, float dz) {
     b.w101 = ff_mul_f(ady, dz);
     b.w011 = ff_mul_f(dxb, dz);
     b.dxdydz = dxdy * dz;
+    // NaN and infinite coordinates, and finite ones beyond the integers, leave fractions
+    // outside [0, 1]: weights are then neither at most 1 nor non-negative
+    const bool unit = dx >= 0.0f && dx <= 1.0f && dy >= 0.0f && dy <= 1.0f && dz >= 0.0f && dz <= 1.0f;
+    b.eps = unit ? 0x1p-40f : INFINITY;
     return b;
 }
 
@@ -206,11 +211,12 @@ __device__ __forceinline__ bool ff_blend8(const FFWeights& b, float c000, float 
     const float S = fabsf(c000) + fabsf(c100) + fabsf(c010) + fabsf(c001) + fabsf(c110) + fabsf(c101) +
                     fabsf(c011) + fabsf(c111);
     if (!(S >= 0x1p-60f && S <= 0x1p+100f)) {  // also NaN / infinite corners
-        // corners that are all +0 (air, a zero field): weights are not negative, so every
-        // product and sum is +0
+        // corners that are all +0 (air, a zero field): weights between 0 and 1 make every
+        // product and sum +0 (a NaN or infinite weight makes NaN)
         out = 0.0f;
-        return (__float_as_uint(c000) | __float_as_uint(c100) | __float_as_uint(c010) | __float_as_uint(c001) |
-                __float_as_uint(c110) | __float_as_uint(c101) | __float_as_uint(c011) | __float_as_uint(c111)) == 0u;
+        const uint32_t bits = __float_as_uint(c000) | __float_as_uint(c100) | __float_as_uint(c010) | __float_as_uint(c001) |
+                              __float_as_uint(c110) | __float_as_uint(c101) | __float_as_uint(c011) | __float_as_uint(c111);
+        return bits == 0u && b.eps < 1.0f;
     }
     FF acc = ff_mul_f(b.w000, c000);
     acc = ff_add(acc, ff_mul_f(b.w100, c100));
@@ -220,7 +226,7 @@ __device__ __forceinline__ bool ff_blend8(const FFWeights& b, float c000, float 
     acc = ff_add(acc, ff_mul_f(b.w101, c101));
     acc = ff_add(acc, ff_mul_f(b.w011, c011));
     acc = ff_add(acc, FF{b.dxdydz * c111, 0.0f});
-    return ff_round_safe(acc, S * 0x1p-40f, out);
+    return ff_round_safe(acc, S * b.eps, out);
 }
 
 // blend8_apply's result in integers, for fractions that are multiples of 2^-5 (grids of

@@ -1,5 +1,7 @@
-"""Displacements and affines that are NaN or infinite: a value that the reference makes NaN
-is NaN, and every other voxel is the reference's bit for bit.
+"""Displacements and affines that are NaN or infinite, over images with and without air
+(zero voxels): a value that the reference makes NaN is NaN, also where all eight corners
+are zero, and every other voxel is the reference's bit for bit.  So are coordinates so far
+beyond the integers that their fractions are far outside [0, 1].
 
 The expected values are the reference's expressions (interp3, warpAffine and
 consistentMappingCL, src/transformations.h:5-26, src/dataCostD.h:278-295,
@@ -108,7 +110,7 @@ def test_expected_values_on_finite_fields():
         assert np.array_equal(got.view(np.uint32), np.asarray(ref).view(np.uint32))
 
 
-@pytest.mark.parametrize("kind", ["dense"])
+@pytest.mark.parametrize("kind", ["zero", "air", "dense"])
 @pytest.mark.parametrize("bad", list(BAD))
 def test_full_fields(bad, kind):
     from deedsbcv_gb300 import api
@@ -122,7 +124,7 @@ def test_full_fields(bad, kind):
     _check(api.warpAffine(dev, AFFINE, *_cuda(f), *DIMS), warp_affine(im, AFFINE, *f, DIMS))
 
 
-@pytest.mark.parametrize("kind", ["dense"])
+@pytest.mark.parametrize("kind", ["zero", "air", "dense"])
 @pytest.mark.parametrize("bad", list(BAD))
 def test_apply_flow(bad, kind):
     from deedsbcv_gb300 import api
@@ -135,7 +137,7 @@ def test_apply_flow(bad, kind):
     _check(api.apply_flow(np.concatenate(f), im, dims=DIMS, X=AFFINE, grid_step=4), ref)
 
 
-@pytest.mark.parametrize("kind", ["dense"])
+@pytest.mark.parametrize("kind", ["zero", "dense"])
 @pytest.mark.parametrize("bad", list(BAD))
 @pytest.mark.parametrize("entry", [0, 3, 6, 11])
 def test_affine(entry, bad, kind):
@@ -152,7 +154,7 @@ def test_affine(entry, bad, kind):
     _check(api.apply_flow(flow, im, dims=DIMS, X=X, grid_step=4), ref)
 
 
-@pytest.mark.parametrize("kind", ["dense"])
+@pytest.mark.parametrize("kind", ["zero", "dense"])
 def test_linear_warp_of_a_degenerate_fit(kind):
     from deedsbcv_gb300 import api
     im = _image(kind, int(np.prod(DIMS)), np.random.default_rng(3))
@@ -160,7 +162,7 @@ def test_linear_warp_of_a_degenerate_fit(kind):
     assert torch.isnan(api.warpAffineLinear(torch.from_numpy(im).cuda(), X, *DIMS)).all()
 
 
-@pytest.mark.parametrize("other", ["smooth"])
+@pytest.mark.parametrize("other", ["zero", "smooth"])
 @pytest.mark.parametrize("bad", list(BAD))
 def test_consistent_mapping(bad, other):
     from deedsbcv_gb300 import api
@@ -197,3 +199,13 @@ def test_soft_warp(bad):
     out.backward(torch.ones_like(out))
     assert not torch.isnan(im.grad).all() and torch.isnan(im.grad).any()
     assert not torch.isnan(field.grad).all() and torch.isnan(field.grad).any()
+
+
+@pytest.mark.parametrize("sign", [-1, 1])
+@pytest.mark.parametrize("beyond", [2.0 ** 21, 2.0 ** 26, 2.0 ** 35, 2.0 ** 90])
+def test_fractions_far_outside(beyond, sign):
+    from deedsbcv_gb300 import api
+    n = int(np.prod(DIMS))
+    rng = np.random.default_rng(int(np.log2(beyond)))
+    im, f = _image("air", n, rng), _field(F32(sign * (2.0 ** 31 + beyond)), n, rng, 0.2)
+    _check(api.warpImageCL(torch.from_numpy(im).cuda(), *_cuda(f), *DIMS), warp_image(im, *f, DIMS))
