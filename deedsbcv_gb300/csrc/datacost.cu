@@ -4,7 +4,7 @@
 //   popcount(F[p] ^ M[clamp(p + d(label))]),
 // d(label) = (ly, lx, lz) * q - q*hw, label = ly + lx*len + lz*len^2.
 //
-// Main path (grid spacing 2..8): the sums run on the tensor cores, as dot products
+// Main path (grid spacing 2..8; few labels an axis: datacost_popc.cu): the sums run on the tensor cores, as dot products
 // of 64 four-bit floats (E2M1) per code whose terms are bit differences less a
 // constant of the fixed code (tmem_st_moving, expand_fixed); a row's sums over its
 // node's sampled columns accumulate exactly in the fp32 accumulators (multiples of
@@ -172,6 +172,7 @@ struct CostPlan {
     int nly;     // y labels per chunk
     int tiles_y, groups, groups_per_cta, splits, chunks;
     int pitch;   // moving rows per class of the split copy
+    double clocks;  // of a column of tiles: all labels of one (x, z), on one SM
 };
 
 // The moving codes with each line's rows split by residue modulo q: class r, entry
@@ -566,7 +567,7 @@ bool cost_plan(int m, int n, int o, int g, int len, int q, CostPlan& best) {
             const double start = 3500.0 + q * NC * c.N * 0.8;
             const double t = (std::max(mma, epi) * len * c.groups + start) * c.tiles_y;
             if (t < best_t) {
-                best_t = t;
+                best_t = c.clocks = t;
                 best = c;
             }
         }
@@ -599,18 +600,71 @@ cudaError_t launch_mma(const uint64_t* d_F, const uint64_t* d_Ms, int m, int n, 
 
 }  // namespace
 
-size_t data_cost_split_count(int m, int n, int o, int g, int hw, int q) {
+namespace {
+// Code pairs a call compares.
+double cost_pairs(int m, int n, int o, int g, int len) {
+    const int S = g > 4 ? 2 : 1, NX = (g + S - 1) / S;
+    return (double)(m / g) * (n / g) * (o / g) * len * len * len * g * NX * NX;
+}
+// The integer kernel is the faster one for few labels an axis, where an MMA step has few
+// columns of labels against a CTA's start and its classes' hand-overs, and at grid 2, whose
+// steps have one or two live classes.  Measured at 192x160x256, integer pipe and tensor cores,
+// each with its copy (the ratio differs little at 113x97x131 and 96x80x112):
+//   3 and 5 labels, always: grid 4, 5 labels, step 1: 466 us, 830; grid 8, 5 labels, step 2:
+//     156, 215;
+//   7 labels: grid 5, step 2: 437, 715; grid 4, step 1: 1083, 1388.  Grids 4, 7 and 8 fill a step of
+//     the tensor cores better at label steps of 3 to 8: grid 4, step 4: 1310, 952 (step 12:
+//     1520, 3770);
+//   grid 2 with steps above 1: 96x80x112, 11 labels, step 2: 0.66 of the time.
+// With 9 labels the sums no longer stay in registers: grid 4, step 1: 5.2 ms, 1.39.
+bool popc_faster(int g, int len, int q) {
+    if (len == 7) return q < 3 || q > 8 || !(g == 4 || g == 7 || g == 8);
+    return len < 7 || (g == 2 && q > 1);
+}
+// Large label steps leave most of a tile's classes almost empty, and one node's samples in
+// registers' reach do better: the generic kernel compares 2 to 4 code pairs a clock and SM
+// whatever the step (21x150x33, grid 5, 11 labels, step 12: 61 us, tensor cores 138;
+// 96x80x112, grid 4, 9 labels, step 28: no tile, 0.63 ms).  A CTA takes 4000 clocks more
+// than cost_plan's start.
+bool generic_faster(int m, int n, int o, int g, int len, const CostPlan& pl) {
+    const double sm_clocks = 152.0, us = 2070.0;
+    const double columns = (double)(n / g) * (o / g) * pl.chunks;
+    const double ctas = columns * pl.tiles_y * pl.splits;
+    const double per_cta = pl.clocks / pl.tiles_y / pl.splits + 4000.0;
+    const double mma = std::max(1.0, ctas / sm_clocks) * per_cta / us;
+    return cost_pairs(m, n, o, g, len) / (2.2 * sm_clocks * us) + 10.0 < mma / 0.85;
+}
+}  // namespace
+
+CostPath data_cost_path(int m, int n, int o, int g, int hw, int q) {
     CostPlan pl;
-    return cost_plan(m, n, o, g, 2 * hw + 1, q, pl) ? (size_t)pl.pitch * q * n * o : 0;
+    const int len = 2 * hw + 1;
+    const bool few = popc_faster(g, len, q);
+    const bool mma = !few && cost_plan(m, n, o, g, len, q, pl);
+    if (few || (len == 7 && !mma)) {
+        // its padded copy must not outweigh the sums (a word costs as much as six pairs), or be
+        // small (8 MB: 4 us)
+        const size_t pad = data_cost_popc_count(m, n, o, g, hw, q);
+        const bool fits = pad > 0 && (pad <= (1u << 20) || 4.0 * pad <= cost_pairs(m, n, o, g, len));
+        return fits ? CostPath::kPopc : CostPath::kGeneric;
+    }
+    return mma && (len == 7 || !generic_faster(m, n, o, g, len, pl)) ? CostPath::kMma : CostPath::kGeneric;
+}
+
+size_t data_cost_scratch_count(int m, int n, int o, int g, int hw, int q) {
+    CostPlan pl;
+    switch (data_cost_path(m, n, o, g, hw, q)) {
+        case CostPath::kPopc: return data_cost_popc_count(m, n, o, g, hw, q);
+        case CostPath::kMma: return cost_plan(m, n, o, g, 2 * hw + 1, q, pl) ? (size_t)pl.pitch * q * n * o : 0;
+        default: return 0;
+    }
 }
 
 cudaError_t launch_data_cost_mma(const uint64_t* d_F, const uint64_t* d_M, uint64_t* d_split, int m, int n, int o,
-                                 int g, int hw, int q, float alpha1, float* d_cost, int* d_err, cudaStream_t s,
-                                 bool* taken) {
+                                 int g, int hw, int q, float alpha1, float* d_cost, int* d_err, cudaStream_t s) {
     CostPlan pl;
     const int len = 2 * hw + 1;
-    *taken = cost_plan(m, n, o, g, len, q, pl);
-    if (!*taken) return cudaSuccess;
+    if (!cost_plan(m, n, o, g, len, q, pl)) return cudaErrorInvalidValue;
     const uint64_t* d_Ms = d_M;
     if (q > 1) {
         k_split_rows<<<dim3((q * pl.pitch + 127) / 128, n, o), 128, 0, s>>>(d_M, d_split, m, n, q * hw, q, pl.pitch);

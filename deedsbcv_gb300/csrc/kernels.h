@@ -45,13 +45,17 @@ cudaError_t launch_mind_ssc(const float* d_im, int m, int n, int o, int qs, cons
                             uint64_t* d_codes, cudaStream_t s);
 cudaError_t launch_data_cost(const uint64_t* d_F, const uint64_t* d_M, int m, int n, int o, int g, int hw, int q,
                              int sy, int sx, int sz, float alpha1, float* d_cost, cudaStream_t s);
-// The tensor-core path (grid spacing 2..8, three labels or more per axis); *taken is
-// false, and nothing is launched, where it does not apply.  d_split: scratch of
-// data_cost_split_count codes (none for a label step of 1).
-size_t data_cost_split_count(int m, int n, int o, int g, int hw, int q);
+// Cost volumes: on the tensor cores, on the integer pipe from padded boxes, or by the
+// generic kernel, which takes any shape.  The first two need a scratch copy of the moving
+// codes, of data_cost_scratch_count words.
+enum class CostPath { kGeneric, kPopc, kMma };
+CostPath data_cost_path(int m, int n, int o, int g, int hw, int q);
+size_t data_cost_scratch_count(int m, int n, int o, int g, int hw, int q);
 cudaError_t launch_data_cost_mma(const uint64_t* d_F, const uint64_t* d_M, uint64_t* d_split, int m, int n, int o,
-                                 int g, int hw, int q, float alpha1, float* d_cost, int* d_err, cudaStream_t s,
-                                 bool* taken);
+                                 int g, int hw, int q, float alpha1, float* d_cost, int* d_err, cudaStream_t s);
+size_t data_cost_popc_count(int m, int n, int o, int g, int hw, int q);  // 0: not for this shape
+cudaError_t launch_data_cost_popc(const uint64_t* d_F, const uint64_t* d_M, uint64_t* d_pad, int m, int n, int o, int g,
+                                  int hw, int q, float alpha1, float* d_cost, int* d_err, cudaStream_t s);
 cudaError_t launch_edge_sad(const float* d_im, int m, int n, int o, int g, float* d_sad, cudaStream_t s);
 // Mean and standard deviation of one or two images in the reference's sequential
 // float semantics (stats.cu): out[2*img + 0 / 1]; im1 unused when nimg is 1.

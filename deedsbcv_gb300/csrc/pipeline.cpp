@@ -251,16 +251,17 @@ void data_cost_params(int g, int q, float alpha, int* sy, int* sx, int* sz, floa
     *alpha1 = (float)(0.5 * alphai / (float)maxsamp);
 }
 
-// Cost volume on the tensor cores where the shape allows it, else by the generic kernel.
+// Cost volume by the kernel that takes the shape in the least time (data_cost_path).
 cudaError_t data_cost_auto(const uint64_t* F, const uint64_t* M, uint64_t* split, int m, int n, int o, int g, int hw,
                            int q, float alpha, float* cost, int* d_err, cudaStream_t s) {
     int sy, sx, sz;
     float alpha1;
     data_cost_params(g, q, alpha, &sy, &sx, &sz, &alpha1);
-    bool taken = false;
-    const cudaError_t e = launch_data_cost_mma(F, M, split, m, n, o, g, hw, q, alpha1, cost, d_err, s, &taken);
-    if (taken || e != cudaSuccess) return e;
-    return launch_data_cost(F, M, m, n, o, g, hw, q, sy, sx, sz, alpha1, cost, s);
+    switch (data_cost_path(m, n, o, g, hw, q)) {
+        case CostPath::kMma: return launch_data_cost_mma(F, M, split, m, n, o, g, hw, q, alpha1, cost, d_err, s);
+        case CostPath::kPopc: return launch_data_cost_popc(F, M, split, m, n, o, g, hw, q, alpha1, cost, d_err, s);
+        default: return launch_data_cost(F, M, m, n, o, g, hw, q, sy, sx, sz, alpha1, cost, s);
+    }
 }
 
 deeds_status check_params(deeds_ctx* ctx, const deeds_params* p, int m, int n, int o) {
@@ -408,7 +409,7 @@ struct PairBuffers {
     uint64_t* c_warp[2];
     float* mind_scr[2];
     float* cost[2];
-    uint64_t* msplit[2];  // moving codes with their rows split by class (launch_data_cost_mma)
+    uint64_t* msplit[2];  // the cost volumes' copy of the moving codes (data_cost_scratch_count)
     float *grid, *kgrid, *cons_scr;  // kgrid: the last result's control-grid field (u | v | w)
     void* stats_scr;  // image statistics (deeds::launch_image_stats)
     float *d_stats, *h_stats;  // mean, std of the fixed and of the affine-warped moving image
@@ -428,7 +429,7 @@ deeds_status acquire_buffers(deeds_ctx* ctx, int m, int n, int o, const deeds_pa
         const size_t sz1 = (size_t)B.m1s[l] * B.n1s[l] * B.o1s[l];
         B.max_sz1 = std::max(B.max_sz1, sz1);
         B.max_cost = std::max(B.max_cost, sz1 * len * len * len);
-        B.max_split = std::max(B.max_split, data_cost_split_count(m, n, o, P->grid[l], P->radius[l], P->quant[l]));
+        B.max_split = std::max(B.max_split, data_cost_scratch_count(m, n, o, P->grid[l], P->radius[l], P->quant[l]));
     }
     B.fix = dbuf<float>(ctx, "fix", sz, &st);
     B.mov = dbuf<float>(ctx, "mov", sz, &st);
@@ -618,7 +619,7 @@ deeds_status deeds_data_cost_dev(deeds_ctx* ctx, const uint64_t* d_F, const uint
         return fail(ctx, DEEDS_ERR_INVALID, "bad grid %d / radius %d / quant %d", g, hw, q);
     CK(cudaSetDevice(ctx->device));
     deeds_status st = DEEDS_OK;
-    uint64_t* split = dbuf<uint64_t>(ctx, "msplit_stage", data_cost_split_count(m, n, o, g, hw, q), &st);
+    uint64_t* split = dbuf<uint64_t>(ctx, "msplit_stage", data_cost_scratch_count(m, n, o, g, hw, q), &st);
     int* d_err = dbuf<int>(ctx, "err_dc_stage", 1, &st);
     if (st) return st;
     cudaStream_t s = (cudaStream_t)stream;
@@ -2133,7 +2134,7 @@ deeds_status deeds_linear_register_dev(deeds_ctx* ctx, const float* d_fixed, con
     for (int l = 0; l < P->levels; l++) {
         const int g = P->grid[l], len = 2 * P->radius[l] + 1;
         max_cost = std::max(max_cost, (size_t)(m / g) * (n / g) * (o / g) * len * len * len);
-        max_split = std::max(max_split, data_cost_split_count(m, n, o, P->grid[l], P->radius[l], P->quant[l]));
+        max_split = std::max(max_split, data_cost_scratch_count(m, n, o, P->grid[l], P->radius[l], P->quant[l]));
     }
     float* fix = dbuf<float>(ctx, "lin_fix", sz, &st);
     float* mov = dbuf<float>(ctx, "lin_mov", sz, &st);
