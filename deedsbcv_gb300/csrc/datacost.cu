@@ -177,12 +177,11 @@ struct CostPlan {
 
 // The moving codes with each line's rows split by residue modulo q: class r, entry
 // b = row r + q b of the line padded by `pad` clamped rows in front.
-__global__ void k_split_rows(const uint64_t* __restrict__ M, uint64_t* __restrict__ Ms, int m, int n, int pad, int q,
-                             int pitch) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void k_split_rows(const uint64_t* __restrict__ M, uint64_t* __restrict__ Ms, int m, int pad, int q, int pitch) {
+    const int e = blockIdx.y * blockDim.x + threadIdx.x;
     if (e >= q * pitch) return;
     const int r = e / pitch, b = e - r * pitch;
-    const int64_t line = blockIdx.y + (int64_t)blockIdx.z * n;
+    const int64_t line = blockIdx.x;  // n o of them: too many for another grid axis
     Ms[line * q * pitch + e] = __ldg(M + line * m + clampi(r + q * b - pad, 0, m - 1));
 }
 
@@ -575,7 +574,7 @@ bool cost_plan(int m, int n, int o, int g, int len, int q, CostPlan& best) {
     if (best_t == 1e300) return false;
     // rows per class: the last tile's rows (beyond the volume too) and the label reach
     best.pitch = q > 1 ? (best.tiles_y * best.tn * g + q - 1) / q + chunks * nly + 2 : 0;
-    if ((uint64_t)std::max(m, q * best.pitch) * n * o >= (1ull << 32)) return false;
+    if ((uint64_t)std::max(m, q * best.pitch) * n * o >= (1ull << 32) || q * best.pitch > 128 * 65535) return false;
     // enough CTAs for several waves of one per SM
     const int64_t cols = (int64_t)best.tiles_y * n1 * o1 * chunks;
     int splits = 1;
@@ -667,8 +666,9 @@ cudaError_t launch_data_cost_mma(const uint64_t* d_F, const uint64_t* d_M, uint6
     if (!cost_plan(m, n, o, g, len, q, pl)) return cudaErrorInvalidValue;
     const uint64_t* d_Ms = d_M;
     if (q > 1) {
-        k_split_rows<<<dim3((q * pl.pitch + 127) / 128, n, o), 128, 0, s>>>(d_M, d_split, m, n, q * hw, q, pl.pitch);
+        k_split_rows<<<dim3(n * o, (q * pl.pitch + 127) / 128), 128, 0, s>>>(d_M, d_split, m, q * hw, q, pl.pitch);
         count_launches(1);
+        if (const cudaError_t e = cudaGetLastError(); e != cudaSuccess) return e;
         d_Ms = d_split;
     }
 #define DEEDS_MMA_ARGS d_F, d_Ms, m, n, o, len, q, pl, alpha1, d_cost, d_err, s

@@ -330,6 +330,7 @@ cudaError_t launch_data_cost_popc(const uint64_t* d_F, const uint64_t* d_M, uint
     if (!popc_plan(m, n, o, g, hw, q, p)) return cudaErrorInvalidValue;
     k_pad_codes<<<dim3((p.mpp + 127) / 128, p.np, p.op), 128, 0, s>>>(d_M, d_pad, m, n, o, q * hw, p.mpp, p.np, p.op);
     count_launches(1);
+    if (const cudaError_t e = cudaGetLastError(); e != cudaSuccess) return e;
 #define DEEDS_POPC_ARGS len, q, d_F, d_pad, m, n, o, len, q, p, alpha1, d_cost, d_err, s
     switch (g) {
         case 2: return launch_width<2>(DEEDS_POPC_ARGS);
