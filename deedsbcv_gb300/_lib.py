@@ -34,6 +34,7 @@ EXPORTS = [
     "deeds_lin_smooth_dev", "deeds_estimate_affine_dev", "deeds_affine_robust", "deeds_affine_warp_segmentation",
     "deeds_fuse_labels_dev", "deeds_multi_atlas",
     "deeds_gz_write", "deeds_gz_read", "deeds_gz_last_error", "deeds_selftest_bounded_waits",
+    "deeds_selftest_cost_volume",
 ]
 NOALLOC_MAX_NODES = 131072
 STAGES = ["mind", "datacost", "mst_edges", "bp_up", "bp_down", "transform", "consistent", "tree_wait", "bp_argmin"]
@@ -176,6 +177,7 @@ def load():
     L.deeds_gz_last_error.argtypes = []
     L.deeds_gz_last_error.restype = C.c_char_p
     L.deeds_selftest_bounded_waits.argtypes = [P, P, P, P]
+    L.deeds_selftest_cost_volume.argtypes = [P, C.c_int, P, P]
     for name in EXPORTS:
         fn = getattr(L, name)
         if name not in ("deeds_default_params", "deeds_destroy", "deeds_last_error", "deeds_version",

@@ -92,21 +92,28 @@ __device__ __forceinline__ void st_shared(uint32_t at, float v) {
     asm volatile("st.shared.f32 [%0], %1;" ::"r"(at), "f"(v) : "memory");
 }
 // Wait for an mbarrier phase with the hardware's own short suspension (a suspend-time
-// hint polls, which took a third of the issue slots here).  Bounded by the number of
-// tries, under a microsecond each: the time a preempted context spends off the GPU
-// does not count.
-constexpr uint32_t kTries = 1u << 22;
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-    const uint32_t at = smem_u32(bar);
-    for (uint32_t i = 0; i < kTries; i++) {
-        uint32_t ok;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-            : "=r"(ok)
-            : "r"(at), "r"(parity)
-            : "memory");
-        if (ok) return true;
-    }
+// hint polls, which took a third of the issue slots here).
+__device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// A wait is bounded by its number of tries (kCostTries, 3.7 us each: a second; the time a
+// preempted context spends off the GPU does not count).
+//
+// A warp that gives up waits for nothing more: producers and epilogues leave their loops, an
+// MMA warp goes through its remaining steps with a limit of 0, issuing what nobody will use
+// (which also ends the producers' waits).  The warps' waits run side by side, so a CTA ends
+// within three bounds of a wait (an epilogue's, then an MMA warp's for the accumulator, then
+// for the MMAs in flight) and sets *err; a CTA that starts after that does nothing.  So a launch
+// that fails ends within about three seconds, whatever its number of tiles.
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t tries) {
+    for (uint32_t i = 0; i < tries; i++)
+        if (mbar_try(bar, parity)) return true;
     return false;
 }
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
@@ -190,11 +197,11 @@ __global__ void k_split_rows(const uint64_t* __restrict__ M, uint64_t* __restric
 template <int G, bool SLIDE>
 __global__ void __launch_bounds__(kCostThreads, 1)
     k_data_cost_mma(const uint64_t* __restrict__ F, const uint64_t* __restrict__ Ms, float* __restrict__ cost, int m,
-                    int n, int o, int len, int q, CostPlan pl, float alpha1, int* __restrict__ err) {
+                    int n, int o, int len, int q, CostPlan pl, float alpha1, uint32_t epi_tries, int* __restrict__ err) {
     constexpr int S = G > 4 ? 2 : 1;  // x and z sampling stride (RAND_SAMPLES=1, src/dataCostD.h:141-155)
     constexpr int NX = (G + S - 1) / S, NZ = NX, NC = NX * NZ;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t b_full[4], b_done[8], b_acc[3], b_free[3], b_turn[2];
+    __shared__ __align__(8) uint64_t b_full[4], b_done[8], b_acc[3], b_free[3], b_turn[2], b_drain[2];
     __shared__ uint32_t s_tmem;
     __shared__ int s_failed;
     const int tid = threadIdx.x, lane = tid & 31;
@@ -232,7 +239,10 @@ __global__ void __launch_bounds__(kCostThreads, 1)
                 mbar_init(&b_acc[i], 1);
                 mbar_init(&b_free[i], 4);
             }
-            for (int i = 0; i < 2; i++) mbar_init(&b_turn[i], 1);
+            for (int i = 0; i < 2; i++) {
+                mbar_init(&b_turn[i], 1);
+                mbar_init(&b_drain[i], 1);
+            }
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
     }
@@ -272,8 +282,7 @@ __global__ void __launch_bounds__(kCostThreads, 1)
     __syncthreads();
     tmem_fence_after();
 
-    const auto wait_done = [&](int t) { return mbar_wait(&b_done[t & 7], (uint32_t)((t >> 3) & 1)); };
-    const auto wait_full = [&](int t) { return mbar_wait(&b_full[t & 3], (uint32_t)((t >> 2) & 1)); };
+    const auto wait_done = [&](int t) { return mbar_wait(&b_done[t & 7], (uint32_t)((t >> 3) & 1), kCostTries); };
     const uint32_t quadrant = (uint32_t)((warp & 3) * 32) << 16;
     const int row = tid & 127;
     const int p = row / pl.R, yb = row - p * pl.R;  // this thread's z offset and moving row
@@ -367,7 +376,7 @@ __global__ void __launch_bounds__(kCostThreads, 1)
         int lx = e, gi = 0;
         while (lx >= len) { lx -= len; gi++; }
         for (int st = e; st < n_steps; st += kEpiGroups) {
-            ok = __all_sync(0xffffffffu, mbar_wait(&b_acc[e], (uint32_t)((st / kEpiGroups) & 1)));
+            ok = __all_sync(0xffffffffu, mbar_wait(&b_acc[e], (uint32_t)((st / kEpiGroups) & 1), epi_tries));
             if (ok) {
                 tmem_fence_after();
 #pragma unroll
@@ -414,13 +423,13 @@ __global__ void __launch_bounds__(kCostThreads, 1)
         const auto issue_steps = [&](auto which) {
         constexpr int e = decltype(which)::value;
         const uint32_t el = elect_one();
+        uint32_t limit = kCostTries;  // 0 after a wait that gave up
         // M = 128, N, E2M1 operands, E8M0 scales, K = 64
         const uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(pl.N >> 3) << 17) | (1u << 23) | (1u << 27);
         // B: K-major without swizzle: 8 x 16 B core matrices, 128 B apart along the
         // rows, N * 16 B apart along K
         const uint32_t blo0 = ((smem_u32(smem_raw) & 0x3ffffu) >> 4) | ((uint32_t)pl.N << 16);
         const uint32_t bhi = 8u | (1u << 14), sf = tmem + kColS;
-        int last = -1;  // the last step committed
         int x = 0, col = 0;  // the step's number in its group, its first ring column
         const auto next = [&]() {
             col += q * USTEP;
@@ -429,21 +438,23 @@ __global__ void __launch_bounds__(kCostThreads, 1)
         };
         if (e) next();
         for (int st = e; st < n_steps; st += 2) {
-            // (A wait that gives up only marks the launch as failed: the warp goes on without a
-            // branch, so that the operands stay in uniform registers and the issue does not stall.)
+            // (A wait that gives up only sets the limit of the waits that follow to 0: with a branch, or
+            // with the issue made to depend on it, the operands leave the uniform registers and the
+            // issue stalls, 1.9 -> 3.4 ms at grid 8.)
             bool in = true;
             // the other warp has seen every tile of its step in place, and its accumulator
             // free (a parity says nothing about the phase before it)
-            if (st >= 1) in = mbar_wait(&b_turn[1 - e], (uint32_t)(((st - 1) >> 1) & 1));
+            if (st >= 1) in = mbar_wait(&b_turn[1 - e], (uint32_t)(((st - 1) >> 1) & 1), limit);
             const int acc = st % kEpiGroups;
-            if (st >= kEpiGroups) in = in && mbar_wait(&b_free[acc], (uint32_t)((st / kEpiGroups - 1) & 1));
+            if (st >= kEpiGroups) in = in && mbar_wait(&b_free[acc], (uint32_t)((st / kEpiGroups - 1) & 1), limit);
             const uint32_t d = tmem + kColD + (uint32_t)(acc * kMaxN);
             ok = ok && in;
             int cj = col;
             uint32_t blo = blo0;
             for (int r = 0; r < q; r++) {
                 const int t = st * q + r;
-                ok = wait_full(t) && ok;
+                limit = ok ? limit : 0u;
+                ok = mbar_wait(&b_full[t & 3], (uint32_t)((t >> 2) & 1), limit) && ok;
                 if (r == q - 1 && lane == 0) mbar_arrive(&b_turn[e]);
                 tmem_fence_after();
                 if (el) {
@@ -466,14 +477,17 @@ __global__ void __launch_bounds__(kCostThreads, 1)
                 cj += NX;
                 cj = cj >= kRingCols ? cj - kRingCols : cj;
                 blo += (uint32_t)NC * (col_bytes >> 4);
-                last = st;
             }
             next();
             next();
         }
-        // no MMA is in flight when the memory is given back: its commits have arrived
-        // (each warp waits for its own last one)
-        if (last >= 0 && !mbar_wait(&b_acc[last % kEpiGroups], (uint32_t)((last / kEpiGroups) & 1))) ok = false;
+        // no MMA is in flight when the memory is given back (a commit covers all MMAs of the
+        // thread that issued them)
+        if (n_steps > e) {
+            if (el) mma_commit(&b_drain[e]);
+            __syncwarp();
+            ok = mbar_wait(&b_drain[e], 0, kCostTries) && ok;
+        }
         };
         if (warp == kMmaWarp) issue_steps(std::integral_constant<int, 0>{});
         else issue_steps(std::integral_constant<int, 1>{});
@@ -586,13 +600,14 @@ bool cost_plan(int m, int n, int o, int g, int len, int q, CostPlan& best) {
 
 template <int G, bool SLIDE>
 cudaError_t launch_mma(const uint64_t* d_F, const uint64_t* d_Ms, int m, int n, int o, int len, int q,
-                       const CostPlan& pl, float alpha1, float* d_cost, int* d_err, cudaStream_t s) {
+                       const CostPlan& pl, float alpha1, float* d_cost, int* d_err, uint32_t epi_tries, cudaStream_t s) {
     const size_t smem = cost_smem(pl, G, q);
     // the same limit on every call: other threads launch the kernel for other sizes
     cudaError_t e = cudaFuncSetAttribute(k_data_cost_mma<G, SLIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
     if (e != cudaSuccess) return e;
     const dim3 grid((unsigned)(pl.tiles_y * (n / G) * (o / G)), (unsigned)pl.splits, (unsigned)pl.chunks);
-    k_data_cost_mma<G, SLIDE><<<grid, kCostThreads, smem, s>>>(d_F, d_Ms, d_cost, m, n, o, len, q, pl, alpha1, d_err);
+    k_data_cost_mma<G, SLIDE>
+        <<<grid, kCostThreads, smem, s>>>(d_F, d_Ms, d_cost, m, n, o, len, q, pl, alpha1, epi_tries, d_err);
     count_launches(1);
     return cudaGetLastError();
 }
@@ -660,7 +675,8 @@ size_t data_cost_scratch_count(int m, int n, int o, int g, int hw, int q) {
 }
 
 cudaError_t launch_data_cost_mma(const uint64_t* d_F, const uint64_t* d_M, uint64_t* d_split, int m, int n, int o,
-                                 int g, int hw, int q, float alpha1, float* d_cost, int* d_err, cudaStream_t s) {
+                                 int g, int hw, int q, float alpha1, float* d_cost, int* d_err, cudaStream_t s,
+                                 uint32_t epi_tries) {
     CostPlan pl;
     const int len = 2 * hw + 1;
     if (!cost_plan(m, n, o, g, len, q, pl)) return cudaErrorInvalidValue;
@@ -671,7 +687,7 @@ cudaError_t launch_data_cost_mma(const uint64_t* d_F, const uint64_t* d_M, uint6
         if (const cudaError_t e = cudaGetLastError(); e != cudaSuccess) return e;
         d_Ms = d_split;
     }
-#define DEEDS_MMA_ARGS d_F, d_Ms, m, n, o, len, q, pl, alpha1, d_cost, d_err, s
+#define DEEDS_MMA_ARGS d_F, d_Ms, m, n, o, len, q, pl, alpha1, d_cost, d_err, epi_tries, s
     switch (g) {
         case 2: return q == 1 ? launch_mma<2, true>(DEEDS_MMA_ARGS) : launch_mma<2, false>(DEEDS_MMA_ARGS);
         case 3: return q == 1 ? launch_mma<3, true>(DEEDS_MMA_ARGS) : launch_mma<3, false>(DEEDS_MMA_ARGS);
@@ -743,7 +759,7 @@ __global__ void k_selftest_mbar_wait(int* status) {
     if (threadIdx.x == 0) {
         mbar_init(&bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        *status = mbar_wait(&bar, 0) ? 2 : 1;
+        *status = mbar_wait(&bar, 0, kCostTries) ? 2 : 1;
     }
 }
 }  // namespace

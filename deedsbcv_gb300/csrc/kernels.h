@@ -51,8 +51,10 @@ cudaError_t launch_data_cost(const uint64_t* d_F, const uint64_t* d_M, int m, in
 enum class CostPath { kGeneric, kPopc, kMma };
 CostPath data_cost_path(int m, int n, int o, int g, int hw, int q);
 size_t data_cost_scratch_count(int m, int n, int o, int g, int hw, int q);
+constexpr uint32_t kCostTries = 1u << 18;  // tries of a wait: about a second (the epilogues' can be set for a self-test)
 cudaError_t launch_data_cost_mma(const uint64_t* d_F, const uint64_t* d_M, uint64_t* d_split, int m, int n, int o,
-                                 int g, int hw, int q, float alpha1, float* d_cost, int* d_err, cudaStream_t s);
+                                 int g, int hw, int q, float alpha1, float* d_cost, int* d_err, cudaStream_t s,
+                                 uint32_t epi_tries = kCostTries);
 size_t data_cost_popc_count(int m, int n, int o, int g, int hw, int q);  // 0: not for this shape
 cudaError_t launch_data_cost_popc(const uint64_t* d_F, const uint64_t* d_M, uint64_t* d_pad, int m, int n, int o, int g,
                                   int hw, int q, float alpha1, float* d_cost, int* d_err, cudaStream_t s);

@@ -2264,4 +2264,32 @@ deeds_status deeds_selftest_bounded_waits(deeds_ctx* ctx, int* sweep_gave_up, in
     return DEEDS_OK;
 }
 
+deeds_status deeds_selftest_cost_volume(deeds_ctx* ctx, int tries, int* error, double* seconds) {
+    if (!ctx) return fail(nullptr, DEEDS_ERR_INVALID, "ctx is NULL");
+    if (tries < 0) return fail(ctx, DEEDS_ERR_INVALID, "tries %d < 0", tries);
+    CK(cudaSetDevice(ctx->device));
+    // steps of 20 classes: an epilogue waits longer than a try for each
+    constexpr int m = 256, n = 64, o = 64, g = 8, hw = 10, q = 20, len = 2 * hw + 1;
+    const size_t sz = (size_t)m * n * o, nc = sz / (g * g * g) * len * len * len;
+    deeds_status st = DEEDS_OK;
+    uint64_t* codes = dbuf<uint64_t>(ctx, "selftest_codes", sz, &st);
+    uint64_t* split = dbuf<uint64_t>(ctx, "msplit_stage", data_cost_scratch_count(m, n, o, g, hw, q), &st);
+    float* cost = dbuf<float>(ctx, "selftest_cost", nc, &st);
+    int* d_err = dbuf<int>(ctx, "err_dc_stage", 1, &st);
+    if (st) return st;
+    cudaStream_t s = ctx->stream;
+    CK(cudaMemsetAsync(codes, 0, sz * sizeof(uint64_t), s));
+    CK(cudaMemsetAsync(d_err, 0, sizeof(int), s));
+    CK(cudaStreamSynchronize(s));
+    const auto t0 = std::chrono::steady_clock::now();
+    CK(launch_data_cost_mma(codes, codes, split, m, n, o, g, hw, q, 1.0f, cost, d_err, s,
+                            tries > 0 ? (uint32_t)tries : kCostTries));
+    int h = 0;
+    CK(cudaMemcpyAsync(&h, d_err, sizeof(h), cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    if (seconds) *seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+    if (error) *error = h;
+    return DEEDS_OK;
+}
+
 }  // extern "C"

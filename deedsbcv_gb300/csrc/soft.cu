@@ -1725,7 +1725,7 @@ __device__ __forceinline__ void red_release_add(int* p, int v) {
     asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-constexpr int kSweepSpinLimit = 1 << 21;  // polls of an L2 round trip each: about a second
+constexpr int kSweepSpinLimit = 1 << 21;  // polls of an L2 round trip each: 0.4 s
 
 // Polls until ready(); gives up after the limit (setting *err) or soon after another
 // thread did, and returns false then (the caller carries on with what it has).

@@ -452,6 +452,12 @@ deeds_status deeds_affine_robust(const float* pts1, const float* pts2, int len, 
  * expired and reported it (the error word for the sweep), *seconds to the time
  * both took.  The context stays usable afterwards. */
 deeds_status deeds_selftest_bounded_waits(deeds_ctx* ctx, int* sweep_gave_up, int* tma_gave_up, double* seconds);
+/* One launch of the tensor-core cost volume (of zero codes) whose epilogue warps give
+ * up a wait after `tries` tries of a few microseconds (0: the production limit, about a
+ * second): *error is the launch's error word (0, or 3 where a wait expired), *seconds its
+ * time.  With few tries an epilogue gives up while the other warps are at work; they then
+ * run into the production limit, and the launch ends. */
+deeds_status deeds_selftest_cost_volume(deeds_ctx* ctx, int tries, int* error, double* seconds);
 
 /* ---------------------------------------------------------------------------
  * Multi-atlas segmentation.  The reference names joint label fusion of several
