@@ -128,6 +128,7 @@ cudaError_t launch_soft_cost_adj(const float* sF, const float* sM, const float* 
                                  float* sMbar, double* dot, int m, int n, int o, int g, int hw, int q, float alpha1,
                                  float eps, cudaStream_t st);
 size_t soft_tree_smem(int len);
+bool soft_tree_needs_bpart(int len);  // whether the backward sweeps use Bpart (sz rows)
 // Tree sweeps are persistent kernels; sweep_mem holds sz + 2 ints (ticket, per-node
 // flags, error word).  The error word must be zeroed before the first sweep and is
 // non-zero afterwards if a bounded wait gave up.

@@ -1601,7 +1601,8 @@ deeds_status soft_issue_backward(deeds_ctx* ctx, const float* d_fixed, const flo
     }
     float* R = dbuf<float>(ctx, "soft_R", L.sz1 * L.len3, &st);
     float* Bbar = dbuf<float>(ctx, "soft_Bbar", L.sz1 * L.len3, &st);
-    float* Bpart = dbuf<float>(ctx, "soft_Bpart", L.sz1 * L.len3, &st);
+    float* Bpart =
+        soft_tree_needs_bpart(2 * p->radius + 1) ? dbuf<float>(ctx, "soft_Bpart", L.sz1 * L.len3, &st) : nullptr;
     float* sFbar = dbuf<float>(ctx, "soft_sFbar", 12 * L.sz, &st);
     float* sMbar = dbuf<float>(ctx, "soft_sMbar", 12 * L.sz, &st);
     float* dbar6 = dbuf<float>(ctx, "soft_dbar6", 6 * L.sz, &st);

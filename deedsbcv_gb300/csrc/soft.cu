@@ -2531,6 +2531,8 @@ cudaError_t launch_soft_cost_adj(const float* sF, const float* sM, const float* 
 // pairs running on other streams.
 constexpr int kSweepCtasPerSm = 2;
 
+// the widths of k_sweep
+bool soft_tree_needs_bpart(int len) { return len <= 9; }
 size_t soft_tree_smem(int len) { return sizeof(float) * (6 * (size_t)len * len * len + 96); }
 
 template <int KIND>
