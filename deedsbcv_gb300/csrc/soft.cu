@@ -1747,8 +1747,9 @@ __device__ __forceinline__ bool bounded_wait_geq(const int* flag, int need, int*
 
 // A row that other nodes of the same sweep wait for is its own flag: it starts as
 // kNotYet in every word, each word is stored once, and a reader polls the words that
-// it uses.  No word depends on another, so nothing has to be ordered.  (The store never
-// writes kNotYet itself: a NaN with just these bits becomes the usual one.)
+// it uses.  No word depends on another, so nothing has to be ordered.  The lanes of a warp
+// see their words at different times and are brought together again behind the poll.
+// (The store never writes kNotYet itself: a NaN with just these bits becomes the usual one.)
 constexpr uint32_t kNotYet = 0xffffffffu;
 
 __device__ __forceinline__ uint32_t ld_word(const float* p) {
@@ -1763,6 +1764,7 @@ __device__ __forceinline__ void st_word(float* p, float v) {
 __device__ __forceinline__ float wait_word(const float* p, int* err) {
     uint32_t v;
     bounded_poll([&] { return (v = ld_word(p)) != kNotYet; }, err);
+    __syncwarp();
     return __uint_as_float(v);
 }
 
@@ -1957,6 +1959,7 @@ __device__ __forceinline__ float wait_children(const SoftTree& t, int c, const N
                 if (i < pre.nch) ok = ok && xs[i] != kNotYet && ms[i] != kNotYet;
             return ok;
         }, err);
+        __syncwarp();
 #pragma unroll
         for (int i = 0; i < kMaxChildren; i++)
             if (i < pre.nch) v += xmin ? __uint_as_float(xs[i]) - __uint_as_float(ms[i]) : __uint_as_float(xs[i]);
@@ -1970,12 +1973,21 @@ __device__ __forceinline__ float wait_children(const SoftTree& t, int c, const N
     return v;
 }
 
+// The block barrier of the sweeps whose lanes poll: it wants a warp's lanes together.  (Lanes
+// that left a poll at different times went on separately.  About one backward pass in a
+// thousand then gave up: a block had gone on to its next node while the words of a row's
+// last warp, 320 to 342 of 343, had never been stored.)
+__device__ __forceinline__ void block_sync() {
+    __syncwarp();
+    __syncthreads();
+}
+
 // Block reductions with one barrier; red is not written again before two barriers.
 template <int W>
 __device__ __forceinline__ float all_max(float v, float* red) {
     v = warp_max(v);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
+    block_sync();
     float r = red[0];
 #pragma unroll
     for (int w = 1; w < W; w++) r = fmaxf(r, red[w]);
@@ -1985,7 +1997,7 @@ template <int W>
 __device__ __forceinline__ float all_sum(float v, float* red) {
     v = warp_add(v);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
+    block_sync();
     float r = red[0];
 #pragma unroll
     for (int w = 1; w < W; w++) r += red[w];
@@ -2006,7 +2018,7 @@ __device__ __forceinline__ float all_lse(float mx, float se, float* rmx, float* 
         rmx[threadIdx.x >> 5] = mx;
         rse[threadIdx.x >> 5] = se;
     }
-    __syncthreads();
+    block_sync();
     float m = -INFINITY, t = 0.0f;
 #pragma unroll
     for (int w = 0; w < W; w++) m = fmaxf(m, rmx[w]);
@@ -2034,7 +2046,7 @@ __global__ void __launch_bounds__(SweepShared<LEN>::W * 32, LEN <= 7 ? 2 : 1)
     const float itau = t.itau;
     for (int turn = 0;; turn ^= 1) {
         if (tid == 0) s_tk[turn] = atomicAdd(st.ticket, 1);
-        __syncthreads();
+        block_sync();
         const int tk = s_tk[turn];
         if (tk >= t.sz) break;
         const int c = ordered[kTopDown ? tk : t.sz - 1 - tk];
@@ -2070,16 +2082,16 @@ __global__ void __launch_bounds__(SweepShared<LEN>::W * 32, LEN <= 7 ? 2 : 1)
             const float r = KIND == kSweepDownAdj ? a.logp[(int64_t)p * L3 + l] + a.M[row] * itau
                                                   : __fmul_rn(-e * a.B[row], itau);
             if (in) sh.x[tid] = r;
-            __syncthreads();
+            block_sync();
             const float t1 = lse_line<LEN, 1>(sh.x + by, ly, itau, sgn, oy);
             if (in) sh.y[tid] = t1;
-            __syncthreads();
+            block_sync();
             const float t2 = lse_line<LEN, LEN>(sh.y + bx, lx, itau, sgn, ox);
             if (in) sh.z[tid] = t2;
-            __syncthreads();
+            block_sync();
             const float t3 = lse_line<LEN, L2>(sh.z + bz, lz, itau, sgn, oz);
             if (in) sh.w[tid] = t3;
-            __syncthreads();
+            block_sync();
             adj_weights<LEN, L2>(wz, t2, sh.w + bz, lz, itau, sgn, oz);
             adj_weights<LEN, LEN>(wx, t1, sh.z + bx, lx, itau, sgn, ox);
             adj_weights<LEN, 1>(wy, r, sh.y + by, ly, itau, sgn, oy);
@@ -2098,10 +2110,10 @@ __global__ void __launch_bounds__(SweepShared<LEN>::W * 32, LEN <= 7 ? 2 : 1)
                 for (int i = 0; i < LEN; i++) f[i] = __fmul_rn(-e * (sh.x[by + i] - bmin), itau);
                 const float t1 = lse_values<LEN>(f, ly, itau, sgn, oy);
                 if (in) sh.y[tid] = t1;
-                __syncthreads();
+                block_sync();
                 const float t2 = lse_line<LEN, LEN>(sh.y + bx, lx, itau, sgn, ox);
                 if (in) sh.z[tid] = t2;
-                __syncthreads();
+                block_sync();
                 const float msg = -t.tau * lse_line<LEN, L2>(sh.z + bz, lz, itau, sgn, oz);
                 if (in) st_word(a.M + row, msg);
                 const float mn = -warp_max(-msg);
@@ -2114,13 +2126,13 @@ __global__ void __launch_bounds__(SweepShared<LEN>::W * 32, LEN <= 7 ? 2 : 1)
             } else {
                 const float x = wait_word(a.logp + (int64_t)p * L3 + l, st.err) + v0 * itau;
                 if (in) sh.x[tid] = x;
-                __syncthreads();
+                block_sync();
                 const float t1 = lse_line<LEN, 1>(sh.x + by, ly, itau, sgn, oy);
                 if (in) sh.y[tid] = t1;
-                __syncthreads();
+                block_sync();
                 const float t2 = lse_line<LEN, LEN>(sh.y + bx, lx, itau, sgn, ox);
                 if (in) sh.z[tid] = t2;
-                __syncthreads();
+                block_sync();
                 r = lse_line<LEN, L2>(sh.z + bz, lz, itau, sgn, oz) - e * v1 * itau;
             }
             const float lp = r - all_lse<W>(in ? r : -INFINITY, in ? 1.0f : 0.0f, sh.red[0], sh.red[1]);
@@ -2140,33 +2152,33 @@ __global__ void __launch_bounds__(SweepShared<LEN>::W * 32, LEN <= 7 ? 2 : 1)
                     sh.x[tid] = h;
                     a.Bpart[row] = -e * itau * h;
                 }
-                __syncthreads();
+                block_sync();
                 const float gz = adj_line<LEN, L2>(wz, sh.x + bz, lz, sgn, oz, t.offbar, dof[2]);
                 if (in) sh.y[tid] = gz;
-                __syncthreads();
+                block_sync();
                 const float gx = adj_line<LEN, LEN>(wx, sh.y + bx, lx, sgn, ox, t.offbar, dof[1]);
                 if (in) sh.z[tid] = gx;
-                __syncthreads();
+                block_sync();
                 const float gy = adj_line<LEN, 1>(wy, sh.z + by, ly, sgn, oy, t.offbar, dof[0]);
                 if (in) st_word(a.R + row, gy);
             }
         } else if (!root) {
             const float x = v0 * itau + wait_word(a.Bbar + (int64_t)p * L3 + l, st.err);
             if (in) sh.x[tid] = x;
-            __syncthreads();
+            block_sync();
             const float gz = adj_line<LEN, L2>(wz, sh.x + bz, lz, sgn, oz, t.offbar, dof[2]);
             if (in) sh.y[tid] = gz;
-            __syncthreads();
+            block_sync();
             const float gx = adj_line<LEN, LEN>(wx, sh.y + bx, lx, sgn, ox, t.offbar, dof[1]);
             if (in) sh.z[tid] = gx;
-            __syncthreads();
+            block_sync();
             const float gy = adj_line<LEN, 1>(wy, sh.z + by, ly, sgn, oy, t.offbar, dof[0]);
             const float b = v1 + e * gy;
             const float mean = all_sum<W>(in ? b : 0.0f, sh.red[0]) / (float)L3;
             if (in) st_word(a.Bbar + row, b - mean);
         }
         if (KIND == kSweepUp && !root) {
-            __syncthreads();
+            block_sync();
             if (tid == 0) {
                 float mn = sh.red[1][0];
 #pragma unroll
@@ -2197,7 +2209,7 @@ __global__ void __launch_bounds__(SweepShared<LEN>::W * 32, LEN <= 7 ? 2 : 1)
                 sh.red[3][warp] = s1;
                 sh.red[4][warp] = s2;
             }
-            __syncthreads();
+            block_sync();
             if (tid < 3) {
                 float s = 0.0f;
                 for (int w = 0; w < W; w++) s += sh.red[2 + tid][w];
