@@ -8,7 +8,7 @@
 // of 64 four-bit floats (E2M1) per code whose terms are bit differences less a
 // constant of the fixed code (tmem_st_moving, expand_fixed); a row's sums over its
 // node's sampled columns accumulate exactly in the fp32 accumulators (multiples of
-// 1/2 of at most 2^11).
+// 1/2; a pair gives at most 56, a slot sums min(q, G) rows of up to 16 columns: at most 7168).
 //
 // A label step of q pairs only rows y of one residue modulo q, so rows are taken
 // by residue class: class r of a tile of tn nodes along y (one x, z) has the fixed
@@ -37,7 +37,7 @@
 // used it reached 7.5.  Reached: 13-20 (the tensor pipe is busy 43 % of the time at
 // grid 8): issuing an MMA takes ~32 clocks and each class ~320 for the hand-overs
 // between the warps.  192x160x256, one direction, grids 8/7/6/5/4 of the default
-// schedule: 1.89 / 1.39 / 1.30 / 1.56 / 1.37 ms, 7.5 ms in all (13.8 ms on the integer
+// schedule: 1.89 / 1.37 / 1.30 / 1.56 / 1.37 ms, 7.5 ms in all (13.8 ms on the integer
 // pipe); a 131x118x141 level of grid 5, radius 4, step 3: 0.65 -> 0.24 ms.
 #include <algorithm>
 #include <type_traits>
@@ -169,7 +169,7 @@ constexpr int kCostThreads = (kMmaWarp + 2) * 32;
 constexpr int kRingCols = 12;  // x columns of operand A in tensor memory
 constexpr int kDCols = 96;     // columns of all accumulators: one per epilogue warpgroup
 constexpr int kEntryPitch = 132;  // entries [slot][128 moving rows]: neighbouring nodes' slots start in different banks
-constexpr uint32_t kColD = 384, kColS = 480;  // tensor memory columns: A ring | 2 accumulators | scales
+constexpr uint32_t kColD = 384, kColS = 480;  // tensor memory columns: A ring | accumulators | scales
 
 // How a level's labels are cut into tiles (cost_plan).
 struct CostPlan {
@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(kCostThreads, 1)
     constexpr int kEpiGroups = epi_groups(SLIDE), kProdGroups = kGroups - kEpiGroups;
     constexpr int kMaxN = kDCols / kEpiGroups;  // slots of a tile at most
     constexpr int USTEP = SLIDE ? 1 : NX;  // new x columns per tile
-    // shared memory: B [class][column][2][N][16 B] | entries [2 warpgroups][N][kEntryPitch] | fixed terms [tn]
+    // shared memory: B [class][column][2][N][16 B] | entries [epilogue warpgroups][N][kEntryPitch] | fixed terms [tn]
     const uint32_t col_bytes = (uint32_t)pl.N * 32u;
     float* entries = reinterpret_cast<float*>(smem_raw + (size_t)q * NC * col_bytes);
     int* s_term = reinterpret_cast<int*>(entries + kEpiGroups * pl.N * kEntryPitch);
@@ -413,6 +413,7 @@ __global__ void __launch_bounds__(kCostThreads, 1)
                 sum_of(x, from, to, term);
                 if (to >= 0 && lz0 + to % len3 / len2 < len) emit(from, to, term);
             }
+            __syncwarp();
             bar_any(1 + e, 128, false);  // the entries are read
             lx += kEpiGroups;
             while (lx >= len) { lx -= len; gi++; }
@@ -493,6 +494,7 @@ __global__ void __launch_bounds__(kCostThreads, 1)
         else issue_steps(std::integral_constant<int, 1>{});
     }
     if (!ok) atomicCAS(err, 0, 3);
+    __syncwarp();  // the lanes left their last waits one by one; barrier and release want them together
     tmem_fence_before();
     __syncthreads();
     if (warp == kMmaWarp) {

@@ -139,6 +139,7 @@ __global__ void __launch_bounds__(256) k_data_cost_popc(const __grid_constant__ 
         if (tid == 0) {
             if (!mbar_wait_bounded(&bars[slot], (uint32_t)((lx >> 1) & 1))) s_ok = 0;
         }
+        __syncwarp();  // the barrier wants the waiting lane's warp together
         __syncthreads();
         if (!s_ok) break;
         if (kFixed && active) {
