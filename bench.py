@@ -40,7 +40,7 @@ G, L, Q = (8, 7, 6, 5, 4), (8, 7, 6, 5, 4), (5, 4, 3, 2, 1)
 METRIC = "pairs/s at 192x160x256 (5 levels)"
 # DRAM bytes (read + write) of one finest-level launch at 192x160x256, from
 # `ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum` captures of the
-# bench workload (profiles/dram_traffic_192x160x256.md, mean of two launches),
+# bench workload (under profiles/; mean of two launches),
 # beside the algorithmic bytes of the same launch as `achieved` counts them
 # (k_bp_up: the 122,880 x 729 float cost volume read and its message rows
 # written; k_data_cost_mma: both code volumes read once, the cost volume written).
@@ -730,12 +730,11 @@ def main():
            "d2h_bytes_per_step": 3 * sz1 * 4, "host_inputs": "pinned"}
 
     # ---- roofline of the dominant stage
-    popc_rate = ctx.popc_rate()
     dc_ms, dc_launches = stages["datacost"]
     mind_ms, mind_launches = stages["mind"]
     pop = popc64_per_pair(shape) * args.steps
-    dc_achieved = pop / (dc_ms / 1000.0) / 1e12 if dc_ms > 0 else None
-    mind_bytes = 152 * sz * mind_calls() * args.steps
+    dc_achieved = pop * 2 * 64 / (dc_ms / 1000.0) / 1e12 if dc_ms > 0 else None
+    mind_bytes = 108 * sz * mind_calls() * args.steps
     peaks = {}
     try:
         with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
@@ -748,30 +747,35 @@ def main():
     mind_roof = {
         "bound": "hbm", "unit": "GB/s", "peak": hbm_peak, "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)",
         "ms_per_call": round(mind_s * 1000, 3),
-        # bytes the four kernels move per voxel: image 4 (+ shifted rows from L2) and six
-        # distance channels 24 written (i pass); 2 x 48 read+write (j, k passes); 24 read
+        # bytes the three kernels move per voxel: image 4 (+ shifted rows from L2) and six
+        # distance channels 24 written (i and j pass); 48 read and written (k pass); 24 read
         # and 8 written (quantise)
-        "achieved": 152 * vox / mind_s / 1e9, "frac": 152 * vox / mind_s / 1e9 / hbm_peak,
+        "achieved": 108 * vox / mind_s / 1e9, "frac": 108 * vox / mind_s / 1e9 / hbm_peak,
         "algorithmic_bytes_per_voxel": 12,
         "note": "one call timed alone; the fused minimum is 12 B/voxel (image in, code out): the sequential "
-                "float prefix sums of the reference's box filter (needed for bit-exact codes) keep the three "
-                "passes separate",
+                "float prefix sums of the reference's box filter (needed for bit-exact codes) keep the k pass "
+                "and the quantiser separate",
         "in_pipeline_achieved": (mind_bytes / (mind_ms / 1000.0) / 1e9) if mind_ms else None,
     }
     iso_pop, iso_s, iso_levels = isolated_data_cost(api, ctx, pair, shape)
-    iso_achieved = iso_pop / iso_s / 1e12
+    # a code pair is a dot product of 64 four-bit floats
+    pair_tflop = 2 * 64 / 1e12
+    fp4_peak = 6.0 * peaks.get("bf16_tflops", 1900.0)
+    iso_achieved = iso_pop * pair_tflop / iso_s
     cost_roof = {
         "kernel": "k_data_cost_mma (Hamming cost volume, one direction, all 5 levels)",
-        "bound": "tensor (4-bit MMA issue and hand-overs)",
+        "bound": "tensor (issue of small 4-bit MMAs, most of whose columns pair rows that no label needs)",
         "achieved": iso_achieved,
-        "peak": popc_rate / 1e12,
-        "unit": "Tpopc64/s",
-        "frac": iso_achieved * 1e12 / popc_rate,
+        "peak": fp4_peak,
+        "unit": "TFLOP/s (4-bit, of code pairs that a label needs)",
+        "frac": iso_achieved / fp4_peak,
         "ms_per_pair": round(2 * iso_s * 1000, 3),
         "levels": iso_levels,
-        "in_pipeline": {"achieved": dc_achieved, "frac": (dc_achieved * 1e12 / popc_rate) if dc_achieved else None,
-                        "note": "popc64 per pair / summed stage time of both direction streams, which share the GPU"},
-        "peak_source": "measured by deeds_measure_popc_rate in this run: a register-only probe of XOR + carry-save + POPC, what the integer pipe does of the same work (the kernel's sums run on the tensor cores)",
+        "in_pipeline": {"achieved": dc_achieved, "frac": (dc_achieved / fp4_peak) if dc_achieved else None,
+                        "note": "code pairs / summed stage time of both direction streams, which share the GPU"},
+        "peak_source": "6 x MEASURED_PEAKS.json bf16_tflops (the ratio of the nominal dense 4-bit and bf16 rates)",
+        "note": "an MMA of N <= 32 columns costs 15 to 33 clocks whatever its size: 25 to 47 needed code pairs a clock and "
+                "SM at most in this form (12 on the integer pipe), 13 to 20 reached",
         "work_per_pair": popc64_per_pair(shape),
         "share_of_gpu_time": dc_ms / gpu_stage_ms if gpu_stage_ms else None,
     }

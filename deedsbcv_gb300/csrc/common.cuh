@@ -100,11 +100,6 @@ __device__ __forceinline__ Corners corners(int y, int x, int z, int m2, int n2, 
 // wherever base + d would be, without overflow.
 __device__ __forceinline__ int displaced(int base, int d, int size) { return base + clampi(d, -size, size); }
 
-__device__ __forceinline__ float sample(const float* __restrict__ v, const Corners& c, const Blend8Weights& b) {
-    return blend8_apply(b, __ldg(v + c.o000), __ldg(v + c.o100), __ldg(v + c.o010), __ldg(v + c.o001),
-                        __ldg(v + c.o110), __ldg(v + c.o101), __ldg(v + c.o011), __ldg(v + c.o111));
-}
-
 // ---- The same blend in float-float, with a proof that it rounds the same way
 //
 // GB300 runs FP64 at a small fraction of its FP32 rate, and the blends above are
@@ -286,7 +281,7 @@ static __device__ __noinline__ float blend8_exact(float dx, float dy, float dz, 
     return blend8_apply(blend8_weights(dx, dy, dz), c000, c100, c010, c001, c110, c101, c011, c111);
 }
 
-// sample() through the float-float evaluation, falling back to the exact one.
+// A sample through the float-float evaluation, falling back to the exact one.
 __device__ __forceinline__ float sample_ff(const float* __restrict__ v, const Corners& c, const FFWeights& w,
                                            float dx, float dy, float dz) {
     const float c000 = __ldg(v + c.o000), c100 = __ldg(v + c.o100), c010 = __ldg(v + c.o010),

@@ -373,7 +373,7 @@ void lin_affine_robust(float* RT, const float* p1, const float* p2, int len, boo
             hb[slot + (size_t)half] = B1[i];
             hb[slot + 2 * (size_t)half] = B2[i];
         };
-        if (median == median) {
+        if (median == median) {  // else no residual compares, and the kept half stays as it was
             // more than half of the points are kept: every point is written to the next slot,
             // which moves on for a kept one, and the last slot gets the last kept point
             int count = 0, last = 0;
@@ -384,10 +384,6 @@ void lin_affine_robust(float* RT, const float* p1, const float* p2, int len, boo
                 last = keep ? i : last;
             }
             put(half - 1, last);
-        } else {
-            int count = 0;
-            for (int i = 0; i < len; i++)
-                if (err[i] <= median) put(std::min(count++, half - 1), i);
         }
         fit(RT, Cols{ha.data(), half}, Cols{hb.data(), half}, rigid);
     }

@@ -434,7 +434,8 @@ __global__ void __launch_bounds__(64) k_quantise(const float* __restrict__ D, ui
     if (LOGTHR) {
         // thresholds -log((c+1.5)/6), c = 0..4: c counts when c < z = 6 exp(-x) - 1.5, so the
         // level is ceil(z), or 0 below.  z from the fast reciprocal and exponential is within
-        // 2^-17 of the z of the quotient and of the float thresholds: relative errors of
+        // 2^-17 of the z of the quotient and of the float thresholds (the reciprocal is normal: a
+        // finite sum leaves a noise below 2^125): relative errors of
         // 2^-22 (exponential), 2^-21.4 (its argument) and 2^-20 (thresholds), with y e^-y <=
         // 0.37, times 6.  One multiply-add places z + 1 at 2^-16 a unit of the mantissa, with
         // the ceiling above the low 16 bits; where those are within 4 of a whole number for
