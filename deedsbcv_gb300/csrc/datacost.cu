@@ -655,15 +655,15 @@ bool generic_faster(int m, int n, int o, int g, int len, const CostPlan& pl) {
 CostPath data_cost_path(int m, int n, int o, int g, int hw, int q) {
     CostPlan pl;
     const int len = 2 * hw + 1;
-    const bool few = popc_faster(g, len, q);
-    const bool mma = !few && cost_plan(m, n, o, g, len, q, pl);
-    if (few || (len == 7 && !mma)) {
+    if (popc_faster(g, len, q)) {
         // its padded copy must not outweigh the sums (a word costs as much as six pairs), or be
         // small (8 MB: 4 us)
         const size_t pad = data_cost_popc_count(m, n, o, g, hw, q);
-        const bool fits = pad > 0 && (pad <= (1u << 20) || 4.0 * pad <= cost_pairs(m, n, o, g, len));
-        return fits ? CostPath::kPopc : CostPath::kGeneric;
+        if (pad > 0 && (pad <= (1u << 20) || 4.0 * pad <= cost_pairs(m, n, o, g, len))) return CostPath::kPopc;
+        // small steps do not fit only where an axis has more lines than a launch grid takes
+        return q <= 8 && cost_plan(m, n, o, g, len, q, pl) ? CostPath::kMma : CostPath::kGeneric;
     }
+    const bool mma = cost_plan(m, n, o, g, len, q, pl);
     return mma && (len == 7 || !generic_faster(m, n, o, g, len, pl)) ? CostPath::kMma : CostPath::kGeneric;
 }
 
